@@ -323,10 +323,9 @@ __device__ __forceinline__ void step(State& st, Slice& s, const Lanes& L, const 
   double factor = controller_factor_sq(err_sq, st.err_prev, st.err_prev2, MDX_E1, MDX_E2, MDX_E3,
                                        MDX_USE_E2, MDX_USE_E3, safe_err);
 #else
-  const double err_norm = sqrt(err_local / MDX_NERR);
-  const bool accept = err_norm <= 1.0 && !isnan(err_norm);
-  double factor = controller_factor(err_norm, st.err_prev, st.err_prev2, MDX_E1, MDX_E2, MDX_E3,
-                                    MDX_USE_E2, MDX_USE_E3, safe_err);
+  bool accept;
+  double factor = controller_factor<6>(err_local, MDX_NERR, st.err_prev, st.err_prev2, MDX_E1, MDX_E2, MDX_E3,
+                                       MDX_USE_E2, MDX_USE_E3, accept, safe_err);
 #endif
   if (accept) {
     st.err_prev2 = st.err_prev;

@@ -171,8 +171,10 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a) {
     const double r = weight(a, st.traj, j) * err_est / scale;
     err_sum += r * r;
   }
-  const double err_norm = sqrt(err_sum / MDX_NERR);
-  const bool accept = err_norm <= 1.0 && !isnan(err_norm);
+  bool accept;
+  double safe_err;
+  double factor = controller_factor<5>(err_sum, MDX_NERR, st.err_prev, st.err_prev2, MDX_E1, MDX_E2, MDX_E3,
+                                       MDX_USE_E2, MDX_USE_E3, accept, safe_err);
 
   double t_new = t;
   if (accept) {
@@ -208,9 +210,6 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a) {
     st.has_fsal = false;
   }
 
-  double safe_err;
-  double factor = controller_factor(err_norm, st.err_prev, st.err_prev2, MDX_E1, MDX_E2, MDX_E3,
-                                    MDX_USE_E2, MDX_USE_E3, safe_err);
   if (accept) {
     st.err_prev2 = st.err_prev;
     st.err_prev = safe_err;
