@@ -380,17 +380,17 @@ def build_source(ode_fn, n_vars: int, n_params: int, options: KernelOptions):
             )
         elif options.sparsity is None:
             structure = dense_jacobian(n_vars)
-            lu_size = n_vars * n_vars
+            lu_size = n_vars * n_vars + n_vars  # the pivots' reciprocals after the factors
             parts.append(f"#define MDX_LU_SIZE {lu_size}")
             parts.append(f"#define MDX_IPIV {n_vars}")
             parts.append('#include "mdx_dense_lu.cuh"')
             parts.append(
                 "template <class LU, class IP> __device__ __forceinline__ void mdx_factorize(LU& lu, IP& ipiv) "
-                "{ mdx::dense_factorize<MDX_NV, MDX_LU_T>(lu, ipiv); }\n"
+                "{ mdx::dense_factorize<MDX_NV, MDX_LU_T, true>(lu, ipiv); }\n"
                 "template <class LU, class IP, class R> __device__ __forceinline__ void mdx_solve(const LU& lu, const IP& ipiv, R& rhs) "
-                "{ mdx::dense_solve<MDX_NV, MDX_SOLVE_T>(lu, ipiv, rhs); }\n"
+                "{ mdx::dense_solve<MDX_NV, MDX_SOLVE_T, true>(lu, ipiv, rhs); }\n"
                 "template <class LU, class IP, class R> __device__ __forceinline__ void mdx_solve_t(const LU& lu, const IP& ipiv, R& rhs) "
-                "{ mdx::dense_solve_t<MDX_NV, MDX_SOLVE_T>(lu, ipiv, rhs); }\n"
+                "{ mdx::dense_solve_t<MDX_NV, MDX_SOLVE_T, true>(lu, ipiv, rhs); }\n"
                 "__device__ __forceinline__ int mdx_diag_slot(int d) { return d * MDX_NV + d; }"
             )
         else:

@@ -302,7 +302,7 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a) {
 #if MDX_FAST
       const double theta = (a.times[st.save_idx] - t) * inv_dt;
 #else
-      const double theta = (a.times[st.save_idx] - t) / dt_use;
+      const double theta = div_by(a.times[st.save_idx] - t, dt_use, inv_dt);
 #endif
       const double theta1 = 1.0 - theta;
 #if MDX_FAST
