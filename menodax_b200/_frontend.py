@@ -105,7 +105,7 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
         from menodax_b200 import autotune
 
         choice = autotune.tune(ode_fn, n_vars, n_params, options, tune_block=tune_block,
-                               tune_team=tune_team, tune_shared=tune_shared, **common)
+                               tune_team=tune_team, tune_shared=tune_shared, tune_registers=tune_team, **common)
         options = autotune.options_for(options, choice)
         problem = get_problem(ode_fn, n_vars, n_params, options)
         mode = choice.mode
@@ -114,6 +114,12 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
             mode = _native.MDX_LAUNCH_PLAIN
             grid_blocks = 0
     else:
+        if launch_mode == "auto" and tune_team and tune_block and not options.team:
+            from menodax_b200 import autotune
+
+            choice = autotune.small_choice(ode_fn, n_vars, n_params, options, n)
+            if choice is not None:
+                options = autotune.options_for(options, choice)
         problem = get_problem(ode_fn, n_vars, n_params, options)
     n_save = int(t_d.shape[0])
     for name, length, lo, hi in problem.hook_tables:

@@ -8,6 +8,7 @@ shapes is a field of ``KernelOptions``, which is also the cache key.
 
 from __future__ import annotations
 
+import functools
 import threading
 from dataclasses import dataclass
 
@@ -21,11 +22,12 @@ from menodax_b200._codegen import (
     emit_sens_coupling,
     lit,
 )
+from menodax_b200 import _cyclic
 from menodax_b200._sparse_direct import MAX_UNROLLED_SUBSTITUTIONS, sparse_lu_for
 from menodax_b200._sparse_direct import emit_cuda as emit_sparse_lu
 from menodax_b200._team import TEAM_SIZES, dense_lda, emit_team_adjoint_functions, emit_team_functions
 from menodax_b200._team import slice_bytes as team_slice_bytes
-from menodax_b200._sparsity import dense_jacobian
+from menodax_b200._sparsity import dense_jacobian, occupancy
 from menodax_b200._trace import trace, trace_array_rhs, trace_hook
 
 TSIT5_EXPONENT = -1.0 / 5.0   # modax/tsit5.py:90
@@ -66,6 +68,9 @@ class KernelOptions:
     # Lanes per trajectory: 0 for the thread-per-trajectory kernels, else 4, 8,
     # 16 or 32 for the team kernel (Rodas5P, no sensitivities, hooks or adjoint).
     team: int = 0
+    # With a team: the cyclic kernel (a block of the state per lane, in registers)
+    # instead of the shared-memory one; see cyclic_lanes for the systems that have it.
+    cyclic: bool = False
     # Tsit5: the stage vectors k1..k6 in shared memory, one column per thread
     # (the reference's "shared" backend, modax/tsit5.py:117-139).
     shared_stages: bool = False
@@ -269,6 +274,84 @@ def _build_team_source(tr, n_vars: int, n_params: int, options: KernelOptions, s
     return "\n".join(parts) + "\n", meta
 
 
+def _cyclic_options(options: KernelOptions) -> bool:
+    """The builds the cyclic kernel covers: plain solves in fast arithmetic with a 32-bit
+    sparse LU.  Its elimination is unpivoted, as the sparse LU's is, in an order of its own, so a
+    dense solve (which pivots) and the reference's arithmetic keep their kernels."""
+    return (options.solver == "rodas5P" and options.fast and options.lu_precision == "fp32"
+            and options.sparsity is not None and options.sparse_code == "auto" and options.ordering == "amd"
+            and options.sens is None and options.save_hook is None and options.array_rhs is None
+            and not options.checkpoint and not options.adjoint and options.save_history)
+
+
+@functools.lru_cache(maxsize=64)
+def _cyclic_layouts(ode_fn, n_vars: int, n_params: int, sparsity):
+    tr = trace(ode_fn, n_vars, n_params)
+    mask = occupancy(sparsity)
+    found = {}
+    for layout in _cyclic.layouts(tr):
+        b = layout.block
+        rows, cols = zip(*[((lane * b + r) % n_vars, (lane * b + offset * b + c) % n_vars)
+                           for r, offset, c in layout.entries for lane in range(layout.lanes)])
+        if mask[list(rows), list(cols)].all():
+            found[layout.lanes] = layout
+    return found
+
+
+def cyclic_lanes(ode_fn, n_vars: int, n_params: int, options: KernelOptions) -> tuple[int, ...]:
+    """The lane counts the cyclic kernel can give a trajectory of this system: those
+    that cut it into equal blocks with the same right-hand side (``_cyclic.analyse``), whose
+    Jacobian the pattern covers.  Empty for any other system or build."""
+    if not _cyclic_options(options):
+        return ()
+    return tuple(sorted(_cyclic_layouts(ode_fn, n_vars, n_params, options.sparsity)))
+
+
+def _build_cyclic_source(ode_fn, tr, n_vars: int, n_params: int, options: KernelOptions):
+    """The cyclic kernel's source: one block's right-hand side, matrix and interior elimination."""
+    lanes, tpb = int(options.team), int(options.threads_per_block)
+    if lanes not in cyclic_lanes(ode_fn, n_vars, n_params, options):
+        raise ValueError(f"the system does not repeat itself over {lanes} lanes, or the build needs another kernel")
+    if tpb % 32:
+        raise ValueError(f"threads_per_block {tpb} is not a whole number of warps")
+    layout = _cyclic_layouts(ode_fn, n_vars, n_params, options.sparsity)[lanes]
+    functions, autonomous = _cyclic.emit_cyclic_functions(tr, layout)
+    e1, e2, e3 = controller_exponents(options)
+    parts = [
+        f"// generated problem source: rodas5P cyclic kernel, n_vars={n_vars}, n_params={n_params}, lanes={lanes}",
+        f"#define MDX_NV {n_vars}",
+        f"#define MDX_NS {n_vars}",
+        f"#define MDX_NP {n_params}",
+        "#define MDX_NSENS 0",
+        f"#define MDX_NERR {lit(float(n_vars))}",
+        "#define MDX_LU_T float",
+        f"#define MDX_TF_INDEX {int(options.tf_index)}",
+        f"#define MDX_E1 {lit(e1)}",
+        f"#define MDX_E2 {lit(e2)}",
+        f"#define MDX_E3 {lit(e3)}",
+        f"#define MDX_USE_E2 {'true' if e2 != 0.0 else 'false'}",
+        f"#define MDX_USE_E3 {'true' if e3 != 0.0 else 'false'}",
+        f"#define MDX_WEIGHTS_RUNTIME {1 if options.runtime_weights else 0}",
+        f"#define MDX_TPB {tpb}",
+        f"#define MDX_MIN_BLOCKS {int(options.min_blocks)}",
+        f"#define MDX_TEAM {lanes}",
+        f"#define MDX_BLOCK {layout.block}",
+        f"#define MDX_SEPARATORS {len(layout.separators)}",
+        f"#define MDX_LANE_PARAMS {len(layout.params)}",
+        f"#define MDX_AUTONOMOUS {1 if autonomous else 0}",
+        '#include "mdx_common.cuh"',
+        "namespace mdx { namespace cyclic {",
+        "typedef MDX_LU_T lu_t;",
+        "// A thread's place in its trajectory, and the warp lanes its team starts at and that hold its neighbours.",
+        "struct Lane { int lane, base, left, right; };",
+        functions,
+        "} }  // namespace mdx::cyclic",
+        '#include "mdx_cyclic.cuh"',
+    ]
+    meta = dict(n_system=n_vars, n_error=n_vars, lu_size=0, sparse=None, hook_tables=[], shared_bytes=0)
+    return "\n".join(parts) + "\n", meta
+
+
 STATIC_SHARED_MAX = 48 * 1024  # a block's static shared memory
 
 
@@ -316,6 +399,8 @@ def build_source(ode_fn, n_vars: int, n_params: int, options: KernelOptions):
         stage_tr = trace_array_rhs(options.array_rhs, tr)
     if options.shared_stages and options.solver != "tsit5":
         raise ValueError("shared_stages places Tsit5's stage vectors; Rodas5P's shared layout is the team kernel")
+    if options.cyclic:
+        return _build_cyclic_source(ode_fn, tr, n_vars, n_params, options)
     if options.team:
         return _build_team_source(tr, n_vars, n_params, options, stage_tr)
     sens = _sens_layout(n_vars, n_params, options.sens)
@@ -493,4 +578,5 @@ def clear_caches() -> None:
     """Drop every compiled problem (``modax/tsit5.py:142-153``)."""
     with _cache_lock:
         _cache.clear()
+    _cyclic_layouts.cache_clear()
     sparse_lu_for.cache_clear()

@@ -33,7 +33,10 @@ warp of trajectories of about the same length finishes together).  When it
 hits the step cap the integrations are long (tens of thousands of steps): the
 plain candidates are ranked by the same capped run, which measures the cost of
 a step with the ensemble resident, and the winner runs as a persistent refill
-launch, since long stiff ensembles have uneven step counts.
+launch, since long stiff ensembles have uneven step counts.  The cost of a step
+does not see the longest trajectories' tail, which more lanes shorten: where the
+cyclic kernel is a candidate, its persistent launches and the winner's are timed
+in full too, while that fits ``BUDGET_S``.
 """
 
 from __future__ import annotations
@@ -49,6 +52,7 @@ from menodax_b200._problem import (
     DENSE_UNROLL_MAX,
     STATIC_SHARED_MAX,
     WIDE_SOLVE_MAX_VARS,
+    cyclic_lanes,
     get_problem,
     team_block_threads,
     tsit5_stage_bytes,
@@ -65,6 +69,11 @@ TEAM_MIN_VARS = 16
 SHARED_STAGES_MAX_VARS = 16   # the reference's bound for its shared Tsit5 backend
 THREAD_MAX_VARS = 128
 WIDE_TUNE_MAX_VARS = 64
+# Threads of a cyclic block: whole trajectories of any lane count, and small enough
+# that registers cost no warp (32, 64 and 128 measured within 3% of one another).
+CYCLIC_BLOCK = 64
+# Lanes that small ensembles are spread over: two warps per scheduler of 148 SMs.
+SMALL_ENSEMBLE_LANES = 148 * 4 * 2 * 32
 
 
 @dataclass(frozen=True)
@@ -75,10 +84,11 @@ class LaunchChoice:
     team: int = 0     # lanes per trajectory; 0 = one thread per trajectory
     shared_stages: bool = False  # Tsit5: stage vectors in shared memory
     wide_solve: bool | None = None  # fast FP32-LU thread kernels: FP64 stage solves; None = by size
+    cyclic: bool = False  # with a team: the cyclic kernel, a block of the state per lane
 
     def describe(self) -> str:
         kind = "plain" if self.mode == _native.MDX_LAUNCH_PLAIN else f"persistent(fill={self.grid_fill})"
-        lanes = f", team of {self.team}" if self.team else ""
+        lanes = f", {'cyclic over' if self.cyclic else 'team of'} {self.team}" if self.team else ""
         stages = ", stages in shared memory" if self.shared_stages else ""
         solves = "" if self.wide_solve is None else (", FP64 solves" if self.wide_solve else ", FP32 solves")
         return f"{kind}, {self.threads_per_block} threads/block{lanes}{stages}{solves}"
@@ -88,7 +98,7 @@ def options_for(options, choice: LaunchChoice):
     """``options`` with the launch choice's block size, team, stage placement and
     solve type."""
     return replace(options, threads_per_block=choice.threads_per_block, team=choice.team,
-                   shared_stages=choice.shared_stages,
+                   shared_stages=choice.shared_stages, cyclic=choice.cyclic,
                    wide_solve=options.wide_solve if choice.wide_solve is None else choice.wide_solve)
 
 
@@ -98,10 +108,11 @@ _cache: dict = {}
 _lock = threading.Lock()
 
 
-def candidates(block_sizes=BLOCK_SIZES, teams=(), shared_blocks=(), shared_default=False, solves=(None,)):
+def candidates(block_sizes=BLOCK_SIZES, teams=(), shared_blocks=(), shared_default=False, solves=(None,), cyclic=()):
     """Thread-kernel launches per block size (and per stage-solve type in
     ``solves``); team launches as ``(team, threads_per_block)`` pairs; Tsit5
-    launches with shared-memory stages per block size in ``shared_blocks``."""
+    launches with shared-memory stages per block size in ``shared_blocks``;
+    cyclic launches per lane count in ``cyclic``."""
     out = []
     for wide in solves:
         for tpb in block_sizes:
@@ -115,6 +126,9 @@ def candidates(block_sizes=BLOCK_SIZES, teams=(), shared_blocks=(), shared_defau
     for team, tpb in teams:
         out.append(LaunchChoice(tpb, _native.MDX_LAUNCH_PLAIN, 0.0, team))
         out.append(LaunchChoice(tpb, _native.MDX_LAUNCH_PERSISTENT, 1.0, team))
+    for lanes in cyclic:
+        out.append(LaunchChoice(CYCLIC_BLOCK, _native.MDX_LAUNCH_PLAIN, 0.0, lanes, cyclic=True))
+        out.append(LaunchChoice(CYCLIC_BLOCK, _native.MDX_LAUNCH_PERSISTENT, 1.0, lanes, cyclic=True))
     return out
 
 
@@ -164,14 +178,54 @@ def _timed_launch(problem, choice, stream, *, n, y0, times, params, weights, dt0
     return e0.elapsed_time(e1) * 1e-3, counters
 
 
+def _fastest_in_full(problem_for, stream, n, max_steps, inputs, choice, buildable):
+    """``choice`` or the cyclic persistent launch that finishes the whole ensemble first;
+    stops timing once the launches so far have taken ``BUDGET_S``."""
+    rivals = [c for c in buildable if c.cyclic and c.mode == _native.MDX_LAUNCH_PERSISTENT and c != choice]
+    best, spent = None, 0.0
+    for candidate in [choice, *rivals]:
+        problem = problem_for(candidate)
+        secs, _ = _timed_launch(problem, candidate, stream, n=n, max_steps=max_steps, **inputs)
+        spent += secs
+        if best is None or secs < best[0]:
+            best = (secs, candidate)
+        if spent + secs > BUDGET_S:
+            break
+    return best[1]
+
+
+def small_choice(ode_fn, n_vars, n_params, options, n) -> LaunchChoice | None:
+    """The launch of an ensemble too small to tune, or ``None`` for the thread kernel's.
+
+    Such an ensemble leaves the device idle, so a cyclic system takes the most lanes
+    a trajectory that still give every scheduler of the device at most two warps (512
+    trajectories on a B200, 4 / 8 / 16 / 32 lanes: the 32-state ring 22.0 / 16.5 / 13.7
+    ms / --, the 64-state Brusselator -- / 0.79 / 0.52 / 0.42 ms; on the shared-memory teams
+    64.4 and 3.5 ms, on threads slower still)."""
+    lanes = cyclic_lanes(ode_fn, n_vars, n_params, options)
+    if not lanes:
+        return None
+    return LaunchChoice(CYCLIC_BLOCK, _native.MDX_LAUNCH_PLAIN, 0.0, _spread(lanes, n), cyclic=True)
+
+
+def _spread(lanes, n: int) -> int:
+    """The most of ``lanes`` that keep ``n`` trajectories within ``SMALL_ENSEMBLE_LANES``."""
+    fitting = [t for t in lanes if t * n <= SMALL_ENSEMBLE_LANES]
+    return max(fitting) if fitting else min(lanes)
+
+
 def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, rtol, atol,
-         max_steps, n_save_hist=None, tune_block=True, tune_team=False, tune_shared=False):
+         max_steps, n_save_hist=None, tune_block=True, tune_team=False, tune_shared=False,
+         tune_registers=False):
     """The fastest launch for this problem on these inputs (device tensors).
 
     With ``tune_block=False`` the block size stays ``options.threads_per_block``
     and only the launch kind and grid are chosen.  With ``tune_team`` the team
     kernel is a candidate too (for systems of ``TEAM_MIN_VARS`` states or more);
     an ``options.team`` already set is kept and only its launch kind is tuned.
+    With ``tune_registers`` so are the kernels that keep a trajectory in its lanes'
+    registers, where they apply: the cyclic kernel, and for dense systems the team
+    kernel's register inverse in place of its shared-memory LU.
     With ``tune_shared`` (Tsit5) the launches with the stage vectors in shared
     memory are candidates beside the register ones; ``options.shared_stages``
     already set keeps them there.
@@ -200,6 +254,11 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
             blocks = ()
         else:
             blocks = BLOCK_SIZES if tune_block else (options.threads_per_block,)
+    cyclic = ()
+    if tune_registers and not options.team:
+        cyclic = cyclic_lanes(ode_fn, n_vars, n_params, options)
+        if cyclic and n_vars >= TEAM_MIN_VARS:
+            blocks, teams = (), ()
     shared_blocks = ()
     if tune_shared and options.solver == "tsit5" and not options.shared_stages and n_vars <= SHARED_STAGES_MAX_VARS:
         shared_blocks = tuple(b for b in blocks if tsit5_stage_bytes(n_vars, b) <= STATIC_SHARED_MAX)
@@ -207,7 +266,7 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
     if (wide_solve_applies(options) and options.wide_solve is None
             and WIDE_SOLVE_MAX_VARS < n_vars <= WIDE_TUNE_MAX_VARS):
         solves = (False, True)
-    cands = candidates(blocks, teams, shared_blocks, options.shared_stages, solves)
+    cands = candidates(blocks, teams, shared_blocks, options.shared_stages, solves, cyclic)
     key = (ode_fn, n_vars, n_params, replace(options, threads_per_block=32, team=0, shared_stages=False), n,
            tuple(cands), max_steps, torch.cuda.get_device_name(y0.device))
     with _lock:
@@ -249,8 +308,11 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
         fill = 1.0 if winner.team else 0.5
         persistent = [c for c in buildable if c.mode == _native.MDX_LAUNCH_PERSISTENT and c.team == winner.team
                       and c.threads_per_block == winner.threads_per_block and c.grid_fill == fill
-                      and c.shared_stages == winner.shared_stages and c.wide_solve == winner.wide_solve]
+                      and c.shared_stages == winner.shared_stages and c.wide_solve == winner.wide_solve
+                      and c.cyclic == winner.cyclic]
         choice = persistent[0] if persistent else winner
+        if cyclic:
+            choice = _fastest_in_full(problem_for, stream, n, max_steps, inputs, choice, buildable)
         with _lock:
             _cache[key] = choice
         return choice
