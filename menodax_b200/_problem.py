@@ -71,6 +71,9 @@ class KernelOptions:
     # With a team: the cyclic kernel (a block of the state per lane, in registers)
     # instead of the shared-memory one; see cyclic_lanes for the systems that have it.
     cyclic: bool = False
+    # With a team and a dense FP32 LU in fast arithmetic: M inverted in the lanes'
+    # registers (kernels/mdx_team_inverse.cuh) instead of factorised in shared memory.
+    inverse: bool = False
     # Tsit5: the stage vectors k1..k6 in shared memory, one column per thread
     # (the reference's "shared" backend, modax/tsit5.py:117-139).
     shared_stages: bool = False
@@ -161,6 +164,20 @@ def team_block_threads(n_vars: int, n_params: int, options: KernelOptions, prefe
     return threads
 
 
+# Matrix entries a lane of the register inverse can keep beside the step's other values.
+INVERSE_MAX_ENTRIES = 128
+
+
+def team_inverse_fits(n_vars: int, options: KernelOptions) -> bool:
+    """Whether a team build can invert its matrix in registers: a plain solve in fast
+    arithmetic with a dense 32-bit matrix, at most 64 rows (their numbers share a word with
+    the pivot search's magnitudes), a lane's rows at most ``INVERSE_MAX_ENTRIES`` entries."""
+    rows = -(-n_vars // options.team) if options.team else n_vars
+    return (bool(options.team) and options.fast and options.lu_precision == "fp32" and options.sparsity is None
+            and not options.checkpoint and not options.adjoint
+            and n_vars <= 64 and rows * n_vars <= INVERSE_MAX_ENTRIES)
+
+
 def _build_team_source(tr, n_vars: int, n_params: int, options: KernelOptions, stage_tr=None):
     """The team kernel's source: class loops for f, -J and df/dt, the matrix in shared memory."""
     if options.solver != "rodas5P":
@@ -171,6 +188,8 @@ def _build_team_source(tr, n_vars: int, n_params: int, options: KernelOptions, s
         raise ValueError("the team kernel integrates the plain system: no forward sensitivities")
     if (options.checkpoint or options.adjoint) and options.sparsity is None:
         raise ValueError("the team kernel's checkpoints and reverse sweep need a sparse LU (a sparsity pattern)")
+    if options.inverse and not team_inverse_fits(n_vars, options):
+        raise ValueError("the register inverse is for fast dense FP32 solves whose rows fit the lanes' registers")
     tpb = int(options.threads_per_block)
     if tpb % 32 or tpb % options.team:
         raise ValueError(f"threads_per_block {tpb} is not a whole number of warps")
@@ -243,6 +262,7 @@ def _build_team_source(tr, n_vars: int, n_params: int, options: KernelOptions, s
         f"#define MDX_MIN_BLOCKS {int(options.min_blocks)}",
         f"#define MDX_TEAM {int(options.team)}",
         f"#define MDX_TEAM_DENSE {1 if dense else 0}",
+        f"#define MDX_TEAM_INVERSE {1 if options.inverse else 0}",
         f"#define MDX_TEAM_LU_SIZE {lu_size}",
         f"#define MDX_TEAM_LU_CLEAR {clear}",
         f"#define MDX_TEAM_SLICE_BYTES {slice_size}",

@@ -55,6 +55,7 @@ from menodax_b200._problem import (
     cyclic_lanes,
     get_problem,
     team_block_threads,
+    team_inverse_fits,
     tsit5_stage_bytes,
     wide_solve_applies,
 )
@@ -85,20 +86,22 @@ class LaunchChoice:
     shared_stages: bool = False  # Tsit5: stage vectors in shared memory
     wide_solve: bool | None = None  # fast FP32-LU thread kernels: FP64 stage solves; None = by size
     cyclic: bool = False  # with a team: the cyclic kernel, a block of the state per lane
+    inverse: bool = False  # with a team, dense: M inverted in registers
 
     def describe(self) -> str:
         kind = "plain" if self.mode == _native.MDX_LAUNCH_PLAIN else f"persistent(fill={self.grid_fill})"
         lanes = f", {'cyclic over' if self.cyclic else 'team of'} {self.team}" if self.team else ""
+        matrix = ", inverse in registers" if self.inverse else ""
         stages = ", stages in shared memory" if self.shared_stages else ""
         solves = "" if self.wide_solve is None else (", FP64 solves" if self.wide_solve else ", FP32 solves")
-        return f"{kind}, {self.threads_per_block} threads/block{lanes}{stages}{solves}"
+        return f"{kind}, {self.threads_per_block} threads/block{lanes}{matrix}{stages}{solves}"
 
 
 def options_for(options, choice: LaunchChoice):
     """``options`` with the launch choice's block size, team, stage placement and
     solve type."""
     return replace(options, threads_per_block=choice.threads_per_block, team=choice.team,
-                   shared_stages=choice.shared_stages, cyclic=choice.cyclic,
+                   shared_stages=choice.shared_stages, cyclic=choice.cyclic, inverse=choice.inverse,
                    wide_solve=options.wide_solve if choice.wide_solve is None else choice.wide_solve)
 
 
@@ -108,11 +111,13 @@ _cache: dict = {}
 _lock = threading.Lock()
 
 
-def candidates(block_sizes=BLOCK_SIZES, teams=(), shared_blocks=(), shared_default=False, solves=(None,), cyclic=()):
+def candidates(block_sizes=BLOCK_SIZES, teams=(), shared_blocks=(), shared_default=False, solves=(None,), cyclic=(),
+               inverse=()):
     """Thread-kernel launches per block size (and per stage-solve type in
     ``solves``); team launches as ``(team, threads_per_block)`` pairs; Tsit5
     launches with shared-memory stages per block size in ``shared_blocks``;
-    cyclic launches per lane count in ``cyclic``."""
+    cyclic launches per lane count in ``cyclic``; ``inverse`` names the teams that
+    invert in registers."""
     out = []
     for wide in solves:
         for tpb in block_sizes:
@@ -124,8 +129,8 @@ def candidates(block_sizes=BLOCK_SIZES, teams=(), shared_blocks=(), shared_defau
         for fill in PERSISTENT_FILL:
             out.append(LaunchChoice(tpb, _native.MDX_LAUNCH_PERSISTENT, fill, 0, True))
     for team, tpb in teams:
-        out.append(LaunchChoice(tpb, _native.MDX_LAUNCH_PLAIN, 0.0, team))
-        out.append(LaunchChoice(tpb, _native.MDX_LAUNCH_PERSISTENT, 1.0, team))
+        out.append(LaunchChoice(tpb, _native.MDX_LAUNCH_PLAIN, 0.0, team, inverse=team in inverse))
+        out.append(LaunchChoice(tpb, _native.MDX_LAUNCH_PERSISTENT, 1.0, team, inverse=team in inverse))
     for lanes in cyclic:
         out.append(LaunchChoice(CYCLIC_BLOCK, _native.MDX_LAUNCH_PLAIN, 0.0, lanes, cyclic=True))
         out.append(LaunchChoice(CYCLIC_BLOCK, _native.MDX_LAUNCH_PERSISTENT, 1.0, lanes, cyclic=True))
@@ -201,16 +206,38 @@ def small_choice(ode_fn, n_vars, n_params, options, n) -> LaunchChoice | None:
     a trajectory that still give every scheduler of the device at most two warps (512
     trajectories on a B200, 4 / 8 / 16 / 32 lanes: the 32-state ring 22.0 / 16.5 / 13.7
     ms / --, the 64-state Brusselator -- / 0.79 / 0.52 / 0.42 ms; on the shared-memory teams
-    64.4 and 3.5 ms, on threads slower still)."""
+    64.4 and 3.5 ms, on threads slower still).  Other systems of ``TEAM_MIN_VARS`` states or
+    more take a team by the same rule: a thread's vectors no longer fit its registers, nor a
+    dense matrix at all (256 trajectories: dense 32 states 94.6 ms on threads, 4.2 on
+    32-lane teams, 1.2 with the register inverse; sparse 64 states 0.75 on threads, 0.18 on
+    32 lanes)."""
     lanes = cyclic_lanes(ode_fn, n_vars, n_params, options)
-    if not lanes:
+    if lanes:
+        return LaunchChoice(CYCLIC_BLOCK, _native.MDX_LAUNCH_PLAIN, 0.0, _spread(lanes, n), cyclic=True)
+    if options.solver != "rodas5P" or n_vars < TEAM_MIN_VARS:
         return None
-    return LaunchChoice(CYCLIC_BLOCK, _native.MDX_LAUNCH_PLAIN, 0.0, _spread(lanes, n), cyclic=True)
+    teams = []
+    for t in team_sizes_for(n_vars):
+        try:
+            team_block_threads(n_vars, n_params, replace(options, team=t), preferred=32)
+        except ValueError:  # a warp's slices exceed a block's shared memory
+            continue
+        teams.append(t)
+    if not teams:
+        return None
+    if team_inverse_fits(n_vars, replace(options, team=teams[-1])):
+        # The inverse gains from lanes for longer: 32 states, 32 / 16 lanes, 1,500
+        # trajectories 2.04 / 2.56 ms, 4,097 5.0 / 5.4.
+        team = _spread(teams, n, 2 * SMALL_ENSEMBLE_LANES)
+    else:
+        team = _spread(teams, n)
+    return LaunchChoice(32, _native.MDX_LAUNCH_PLAIN, 0.0, team,
+                        inverse=team_inverse_fits(n_vars, replace(options, team=team)))
 
 
-def _spread(lanes, n: int) -> int:
-    """The most of ``lanes`` that keep ``n`` trajectories within ``SMALL_ENSEMBLE_LANES``."""
-    fitting = [t for t in lanes if t * n <= SMALL_ENSEMBLE_LANES]
+def _spread(lanes, n: int, most: int = SMALL_ENSEMBLE_LANES) -> int:
+    """The widest of ``lanes`` that keep ``n`` trajectories within ``most`` lanes in all."""
+    fitting = [t for t in lanes if t * n <= most]
     return max(fitting) if fitting else min(lanes)
 
 
@@ -259,6 +286,9 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
         cyclic = cyclic_lanes(ode_fn, n_vars, n_params, options)
         if cyclic and n_vars >= TEAM_MIN_VARS:
             blocks, teams = (), ()
+    inverse = ()
+    if tune_registers:
+        inverse = tuple(t for t, _ in teams if team_inverse_fits(n_vars, replace(options, team=t)))
     shared_blocks = ()
     if tune_shared and options.solver == "tsit5" and not options.shared_stages and n_vars <= SHARED_STAGES_MAX_VARS:
         shared_blocks = tuple(b for b in blocks if tsit5_stage_bytes(n_vars, b) <= STATIC_SHARED_MAX)
@@ -266,7 +296,7 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
     if (wide_solve_applies(options) and options.wide_solve is None
             and WIDE_SOLVE_MAX_VARS < n_vars <= WIDE_TUNE_MAX_VARS):
         solves = (False, True)
-    cands = candidates(blocks, teams, shared_blocks, options.shared_stages, solves, cyclic)
+    cands = candidates(blocks, teams, shared_blocks, options.shared_stages, solves, cyclic, inverse)
     key = (ode_fn, n_vars, n_params, replace(options, threads_per_block=32, team=0, shared_stages=False), n,
            tuple(cands), max_steps, torch.cuda.get_device_name(y0.device))
     with _lock:
@@ -309,7 +339,7 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
         persistent = [c for c in buildable if c.mode == _native.MDX_LAUNCH_PERSISTENT and c.team == winner.team
                       and c.threads_per_block == winner.threads_per_block and c.grid_fill == fill
                       and c.shared_stages == winner.shared_stages and c.wide_solve == winner.wide_solve
-                      and c.cyclic == winner.cyclic]
+                      and c.cyclic == winner.cyclic and c.inverse == winner.inverse]
         choice = persistent[0] if persistent else winner
         if cyclic:
             choice = _fastest_in_full(problem_for, stream, n, max_steps, inputs, choice, buildable)

@@ -70,6 +70,10 @@ struct Slice {
 };
 static_assert(sizeof(Slice) == MDX_TEAM_SLICE_BYTES, "host and device disagree on the slice layout");
 
+#ifndef MDX_TEAM_INVERSE
+#define MDX_TEAM_INVERSE 0
+#endif
+
 struct Lanes {
   int lane;       // lane within the team
   unsigned mask;  // the team's lanes within the warp
@@ -115,6 +119,17 @@ __device__ __forceinline__ double weight(const MdxSolveArgs& a, int traj, int j)
 #endif
 }
 
+}  // namespace team
+}  // namespace mdx
+
+#if MDX_TEAM_INVERSE
+#include "mdx_team_inverse.cuh"
+#endif
+
+namespace mdx {
+namespace team {
+
+#if !MDX_TEAM_INVERSE
 __device__ __forceinline__ void factorize(Slice& s, const Lanes& L) {
 #if MDX_TEAM_DENSE
 #if MDX_FAST
@@ -150,6 +165,7 @@ __device__ __noinline__ void solve(Slice& s, lu_t* x, const Lanes L) {
   __syncwarp(L.mask);
 #endif
 }
+#endif  // !MDX_TEAM_INVERSE
 
 __device__ __forceinline__ void init(State& st, Slice& s, const Lanes& L, const MdxSolveArgs& a, int traj) {
   st.traj = traj;
@@ -197,36 +213,48 @@ __device__ __forceinline__ bool running(const State& st, const MdxSolveArgs& a) 
   return st.save_idx < a.n_save && st.t < st.tf_local && st.n_steps < a.max_steps;
 }
 
-// Stage S's right-hand side into k[S] (rounded to the LU type), then the solve.
+// Component j of stage S's right-hand side.
+template <int S>
+__device__ __forceinline__ double stage_value(const Slice& s, int j, double dt_use, double inv_dt) {
+  if constexpr (S == 0) {
+#if MDX_TEAM_AUTONOMOUS
+    return s.f[j];
+#else
+    return s.f[j] + dt_use * coef_d(0) * s.dT[j];
+#endif
+  } else {
+    double acc = coef_c(S, 0) * (double)s.k[0][j];
+#pragma unroll
+    for (int m = 1; m < S; ++m) acc += coef_c(S, m) * (double)s.k[m][j];
+#if !MDX_TEAM_AUTONOMOUS
+    if constexpr (coef_d(S) != 0.0) return s.f[j] + dt_use * coef_d(S) * s.dT[j] + acc * inv_dt;
+#endif
+    return s.f[j] + acc * inv_dt;
+  }
+}
+
+// Stage S: its right-hand side (rounded to the LU type), then the solve, into k[S].
+#if MDX_TEAM_INVERSE
+template <int S>
+__device__ __forceinline__ void stage(Slice& s, const Inverse& m, const Lanes& L, double dt_use, double inv_dt) {
+  lu_t b[ROWS];
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    const int j = L.lane + q * MDX_TEAM;
+    b[q] = j < MDX_NV ? (lu_t)stage_value<S>(s, j, dt_use, inv_dt) : (lu_t)0;
+  }
+  apply(s, m, b, s.k[S], L);
+}
+#define MDX_TEAM_STAGE(S) stage<S>(s, inverse, L, dt_use, inv_dt)
+#else
+#define MDX_TEAM_STAGE(S) stage<S>(s, L, dt_use, inv_dt)
 template <int S>
 __device__ __forceinline__ void stage(Slice& s, const Lanes& L, double dt_use, double inv_dt) {
-  for (int j = L.lane; j < MDX_NV; j += MDX_TEAM) {
-    double value;
-    if constexpr (S == 0) {
-#if MDX_TEAM_AUTONOMOUS
-      value = s.f[j];
-#else
-      value = s.f[j] + dt_use * coef_d(0) * s.dT[j];
-#endif
-    } else {
-      double acc = coef_c(S, 0) * (double)s.k[0][j];
-#pragma unroll
-      for (int m = 1; m < S; ++m) acc += coef_c(S, m) * (double)s.k[m][j];
-#if !MDX_TEAM_AUTONOMOUS
-      if constexpr (coef_d(S) != 0.0) {
-        value = s.f[j] + dt_use * coef_d(S) * s.dT[j] + acc * inv_dt;
-      } else {
-        value = s.f[j] + acc * inv_dt;
-      }
-#else
-      value = s.f[j] + acc * inv_dt;
-#endif
-    }
-    s.k[S][j] = (lu_t)value;
-  }
+  for (int j = L.lane; j < MDX_NV; j += MDX_TEAM) s.k[S][j] = (lu_t)stage_value<S>(s, j, dt_use, inv_dt);
   __syncwarp(L.mask);
   solve(s, s.k[S], L);
 }
+#endif
 
 template <int S>
 __device__ __forceinline__ void advance(Slice& s, const Lanes& L) {
@@ -273,31 +301,36 @@ __device__ __forceinline__ void step(State& st, Slice& s, const Lanes& L, const 
   __syncwarp(L.mask);
   for (int d = L.lane; d < MDX_NV; d += MDX_TEAM) s.lu[mdx_team_diag_slot(d)] += (lu_t)dtgamma_inv;
   __syncwarp(L.mask);
+#if MDX_TEAM_INVERSE
+  Inverse inverse;
+  invert(s, inverse, L);
+#else
   factorize(s, L);
+#endif
 
   rhs(s, L, s.y, t);
-  stage<0>(s, L, dt_use, inv_dt);
+  MDX_TEAM_STAGE(0);
   advance<0>(s, L);
   rhs(s, L, s.u, t + coef_ct(0) * dt_use);
-  stage<1>(s, L, dt_use, inv_dt);
+  MDX_TEAM_STAGE(1);
   advance<1>(s, L);
   rhs(s, L, s.u, t + coef_ct(1) * dt_use);
-  stage<2>(s, L, dt_use, inv_dt);
+  MDX_TEAM_STAGE(2);
   advance<2>(s, L);
   rhs(s, L, s.u, t + coef_ct(2) * dt_use);
-  stage<3>(s, L, dt_use, inv_dt);
+  MDX_TEAM_STAGE(3);
   advance<3>(s, L);
   rhs(s, L, s.u, t + coef_ct(3) * dt_use);
-  stage<4>(s, L, dt_use, inv_dt);
+  MDX_TEAM_STAGE(4);
   advance<4>(s, L);
   rhs(s, L, s.u, t_end);
-  stage<5>(s, L, dt_use, inv_dt);
+  MDX_TEAM_STAGE(5);
   accumulate(s, L, 5);
   rhs(s, L, s.u, t_end);
-  stage<6>(s, L, dt_use, inv_dt);
+  MDX_TEAM_STAGE(6);
   accumulate(s, L, 6);
   rhs(s, L, s.u, t_end);
-  stage<7>(s, L, dt_use, inv_dt);
+  MDX_TEAM_STAGE(7);
 
   // Weighted RMS of k8 (modax/rodas5P.py:903-911): scaled terms by component on
   // the owning lanes, then the sum of squares in component order on every lane.
