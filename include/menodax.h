@@ -206,6 +206,14 @@ int mdx_solve_persistent_noalloc(mdx_plan* plan, const mdx_solve_desc* desc, voi
 /* Launch the discrete-adjoint reverse pass on `stream` (MDX_PLAN_ADJOINT plans). */
 int mdx_grad(mdx_plan* plan, const mdx_grad_desc* desc, void* stream);
 
+/* The visiting order of a persistent launch (mdx_solve_desc.order): a permutation
+ * of 0..n-1 by descending step count, from `steps` (n ints on the device, such as a
+ * solve's loop_steps) into `order`.  Step counts below 256 are told apart exactly, larger
+ * ones to one part in 128, equal ones in no particular order.  `workspace` is device memory of at
+ * least mdx_order_workspace_size bytes, free again when the stream is past the call. */
+int mdx_order_workspace_size(size_t* bytes);
+int mdx_order_longest_first(const int* steps, int n, int* order, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Measured FMA throughput of the current device's CUDA cores, in FLOP/s
  * (an FMA counts two): the roofline denominator of the ensemble kernels, which
  * are bound by FP64/FP32 issue rather than HBM or the tensor cores.  No

@@ -95,6 +95,11 @@ def pick_device(*tensors):
     return torch.device("cuda", torch.cuda.current_device())
 
 
+def stream_key(device):
+    """What tells the current stream apart in a cache of device tensors that its launches read."""
+    return getattr(torch.cuda.current_stream(device), "cuda_stream", None)
+
+
 def to_device(t, device):
     if t is None:
         return None

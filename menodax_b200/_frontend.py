@@ -19,6 +19,7 @@ from menodax_b200._ensemble import (
     normalize_y0_params,
     pick_device,
     solver_stats,
+    stream_key,
     to_device,
 )
 from menodax_b200._problem import KernelOptions, get_problem
@@ -27,8 +28,8 @@ from menodax_b200.autotune import longest_first
 LAUNCH_MODES = ("auto", "plain", "persistent")
 
 # Per problem (the compiled options, ensemble size, save times, tolerances and
-# step cap): the trajectories of the last persistent launch, most attempted
-# steps first.  The next persistent launch of the same problem takes them in that
+# step cap) and stream (an order is read on the stream that wrote it): the
+# trajectories of the last persistent launch, most attempted steps first.  The next persistent launch of the same problem takes them in that
 # order, so the long integrations start in the grid's first wave instead of
 # setting the makespan from a late one (the 64-state Brusselator's 16,384
 # trajectories 16.9 -> 15.0 ms, the 32-state Van der Pol ring's 32,768 7.5 ->
@@ -142,7 +143,7 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
     order_key = None
     if mode == _native.MDX_LAUNCH_PERSISTENT:
         order_key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol),
-                     int(max_steps), int(grid_blocks))
+                     int(max_steps), int(grid_blocks), stream_key(device))
         order = _order_hint.get(order_key)
         if order is not None and (order.device != device or order.numel() != n):
             order = None

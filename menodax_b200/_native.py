@@ -43,6 +43,7 @@ EXPORTED = (
     "mdx_compile", "mdx_free", "mdx_plan_create", "mdx_plan_destroy", "mdx_workspace_size",
     "mdx_occupancy", "mdx_solve", "mdx_grad", "mdx_last_error", "mdx_version",
     "mdx_measure_fma_peak", "mdx_solve_persistent_noalloc", "mdx_checkpoint_size",
+    "mdx_order_workspace_size", "mdx_order_longest_first",
 )
 
 
@@ -91,7 +92,7 @@ class GradDesc(ctypes.Structure):
 
 def _library_sources():
     return [CSRC / "mdx_runtime.cpp", CSRC / "mdx_peak.cu", CSRC / "mdx_noalloc.cu",
-            CSRC / "mdx_internal.h", KERNEL_DIR / "mdx_args.h", INCLUDE_DIR / "menodax.h"]
+            CSRC / "mdx_order.cu", CSRC / "mdx_internal.h", KERNEL_DIR / "mdx_args.h", INCLUDE_DIR / "menodax.h"]
 
 
 def build_library(force: bool = False) -> Path:
@@ -104,7 +105,7 @@ def build_library(force: bool = False) -> Path:
     cmd = [
         str(CUDA_HOME / "bin" / "nvcc"), "-O2", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC",
         "-Xcompiler", "-Wall", f"-I{CUDA_HOME / 'include'}", str(CSRC / "mdx_runtime.cpp"), str(CSRC / "mdx_peak.cu"),
-        str(CSRC / "mdx_noalloc.cu"),
+        str(CSRC / "mdx_noalloc.cu"), str(CSRC / "mdx_order.cu"),
         "-o", str(LIB_PATH), f"-L{CUDA_HOME / 'lib64'}", "-lnvrtc", "-ldl",
         f"-Xlinker=-rpath,{CUDA_HOME / 'lib64'}",
     ]
@@ -147,6 +148,9 @@ def lib():
         L.mdx_last_error.argtypes = [ctypes.c_char_p, ctypes.c_size_t]
         L.mdx_version.restype = ctypes.c_char_p
         L.mdx_solve_persistent_noalloc.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveDesc), ctypes.c_void_p]
+        L.mdx_order_workspace_size.argtypes = [ctypes.POINTER(ctypes.c_size_t)]
+        L.mdx_order_longest_first.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,
+                                              ctypes.c_size_t, ctypes.c_void_p]
         L.mdx_measure_fma_peak.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
         _lib = L
         return _lib
@@ -157,6 +161,18 @@ def measure_fma_peak(double_precision: bool = True) -> float:
     out = ctypes.c_double()
     check(lib().mdx_measure_fma_peak(1 if double_precision else 0, ctypes.byref(out)), "mdx_measure_fma_peak")
     return out.value
+
+
+def order_workspace_size() -> int:
+    out = ctypes.c_size_t()
+    check(lib().mdx_order_workspace_size(ctypes.byref(out)), "mdx_order_workspace_size")
+    return out.value
+
+
+def order_longest_first(steps: int, n: int, order: int, workspace: int, nbytes: int, stream: int) -> None:
+    """``mdx_order_longest_first`` on device addresses, in the current context."""
+    check(lib().mdx_order_longest_first(steps, n, order, workspace, nbytes, ctypes.c_void_p(stream)),
+          "mdx_order_longest_first")
 
 
 def last_error() -> str:

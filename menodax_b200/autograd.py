@@ -36,7 +36,7 @@ from dataclasses import replace
 import torch
 
 from menodax_b200 import _native, autotune
-from menodax_b200._ensemble import initial_step, launch, pick_device, solver_stats
+from menodax_b200._ensemble import initial_step, launch, pick_device, solver_stats, stream_key
 from menodax_b200._problem import get_problem
 
 # Checkpoint capacity (accepted steps per trajectory) and stride last used per
@@ -112,12 +112,6 @@ def _as_double(x, device):
     if isinstance(x, torch.Tensor):
         return x.to(device=device, dtype=torch.float64)
     return torch.as_tensor(x, dtype=torch.float64, device=device)
-
-
-def _longest_first(accepted):
-    """Trajectory indices by descending step count, as the int32 visiting order
-    the persistent launch takes."""
-    return torch.argsort(accepted, descending=True, stable=True).to(torch.int32)
 
 
 def _forward_blocks(problem, n: int, fill: float = 0.5) -> int:
@@ -215,7 +209,7 @@ class _EnsembleSolve(torch.autograd.Function):
             # First call for this problem: count the accepted steps with a plain solve.
             _, counters = launch(problems["plain"], grid_blocks=_forward_blocks(problems["plain"], n), **kw)
             capacity = max(1, int(counters[0].max().item()) if n else 1)
-            order = _longest_first(counters[0])
+            order = autotune.longest_first(counters[0])
         while True:
             stride = choose_stride(n, problems["plain"].n_vars, capacity, y0.device)
             # Keep the last call's stride when memory still allows it: the same
@@ -235,7 +229,7 @@ class _EnsembleSolve(torch.autograd.Function):
             capacity = int(needed * 1.1) + 8
             del ckpt
         _remember(_capacity_hint, key, (max(needed + 8, int(needed * 1.1)), stride))
-        _remember(_order_hint, key, _longest_first(counters[0]))
+        _remember(_order_hint, key, autotune.longest_first(counters[0]))
         last_checkpoint.update(stride=stride, capacity=capacity, bytes=nbytes, forward_fill=fill)
         ctx.problem = problem
         ctx.capacity = capacity
@@ -286,7 +280,7 @@ class _EnsembleSolve(torch.autograd.Function):
         # Longest reverse sweeps first: the reverse kernel's registers leave room
         # for only part of a large ensemble at once, and a long trajectory that
         # started in a later wave would set the makespan.
-        order = torch.argsort(ckpt_count, descending=True, stable=True).to(torch.int32)
+        order = autotune.longest_first(ckpt_count)
         chunk = reverse_chunk(problem, n)
         with torch.cuda.device(params.device):
             for first in range(0, n, chunk):
@@ -444,7 +438,8 @@ def solve_with_grad(ode_fn, y0, t_span, params, options, *, rtol, atol, first_st
         keep[list(int(c) for c in sens_param_columns)] = 1.0
         p_t = _ColumnMask.apply(p_t, keep)
     problems = _Problems(ode_fn, n_vars, n_params, replace(options, runtime_weights=False))
-    key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol))
+    key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol),
+           stream_key(device))
     hist, counters = _EnsembleSolve.apply(y0_t, p_t, times, problems, initial_step(first_step), rtol,
                                           atol, max_steps, key)
     if return_stats:

@@ -43,6 +43,7 @@ from __future__ import annotations
 
 import threading
 from dataclasses import dataclass, replace
+from functools import lru_cache
 
 import torch
 
@@ -164,9 +165,25 @@ def streams_to_host(choice: LaunchChoice) -> bool:
 
 
 def longest_first(loop_steps: torch.Tensor) -> torch.Tensor:
-    """The int32 visiting order of a persistent launch: trajectories by
-    descending attempted steps (stable, so ties keep index order)."""
-    return torch.argsort(loop_steps, descending=True, stable=True).to(torch.int32)
+    """The int32 visiting order of a persistent launch: trajectories by descending
+    attempted steps.  On the GPU the native counting sort (``mdx_order_longest_first``: equal
+    counts in no particular order, counts of 256 and more to one part in 128), on the
+    current stream."""
+    if not loop_steps.is_cuda:
+        return torch.argsort(loop_steps, descending=True, stable=True).to(torch.int32)
+    device = loop_steps.device
+    steps = loop_steps.to(torch.int32).contiguous()
+    order = torch.empty(steps.shape, dtype=torch.int32, device=device)
+    scratch = torch.empty(_order_workspace(), dtype=torch.uint8, device=device)
+    with torch.cuda.device(device):
+        _native.order_longest_first(steps.data_ptr(), steps.numel(), order.data_ptr(), scratch.data_ptr(),
+                                    scratch.numel(), torch.cuda.current_stream(device).cuda_stream)
+    return order
+
+
+@lru_cache(maxsize=1)
+def _order_workspace() -> int:
+    return _native.order_workspace_size()
 
 
 def _timed_launch(problem, choice, stream, *, n, y0, times, params, weights, dt0, rtol, atol, max_steps,

@@ -29,7 +29,7 @@ import numpy as np
 import torch
 
 from menodax_b200 import _native, autotune
-from menodax_b200._ensemble import initial_step, launch, normalize_y0_params, pick_device, to_device
+from menodax_b200._ensemble import initial_step, launch, normalize_y0_params, pick_device, stream_key, to_device
 from menodax_b200._problem import KernelOptions, get_problem
 
 # Per joint-solve problem: the trajectories of the last call, longest first (by
@@ -148,7 +148,8 @@ def solve(solver, ode_fn, y0, t_span, params, *, wrt_y0=True, wrt_params=True,
     # stiff Van der Pol gradients of 65,536 trajectories: 324 ms plain, 207 ms
     # persistent, 163 ms persistent longest first; the same gradients bit for
     # bit).
-    key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol))
+    key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol),
+           stream_key(device))
     order = _order_hint.get(key)
     if order is not None and (order.device != device or order.numel() != n):
         order = None
@@ -158,7 +159,7 @@ def solve(solver, ode_fn, y0, t_span, params, *, wrt_y0=True, wrt_params=True,
                             max_steps=max_steps, mode=_native.MDX_LAUNCH_PERSISTENT,
                             grid_blocks=autotune.grid_blocks(problem, choice, n), order=order)
     _order_hint.pop(key, None)
-    _order_hint[key] = torch.argsort(counters[0], descending=True, stable=True).to(torch.int32)
+    _order_hint[key] = autotune.longest_first(counters[0])
     while len(_order_hint) > ORDER_HINT_PROBLEMS:
         _order_hint.pop(next(iter(_order_hint)))
     state, sens = split_augmented(hist, spec)
