@@ -128,6 +128,16 @@ def wide_solve_applies(options: KernelOptions) -> bool:
             and options.lu_precision == "fp32")
 
 
+# Dense systems up to this size invert their matrix in double by cofactors where they
+# would solve in double against FP32 factors (kernels/mdx_dense_lu.cuh, closed_inverse).
+CLOSED_INVERSE_MAX = 3
+
+
+def closed_inverse(options: KernelOptions, n_vars: int) -> bool:
+    return (options.sparsity is None and options.sens is None and n_vars <= CLOSED_INVERSE_MAX
+            and wide_solve(options, n_vars))
+
+
 def wide_solve(options: KernelOptions, n_vars: int) -> bool:
     """Whether a thread-kernel Rodas5P build solves its stages in double against
     FP32 factors: ``options.wide_solve`` when set, else for systems of at most
@@ -432,6 +442,9 @@ def build_source(ode_fn, n_vars: int, n_params: int, options: KernelOptions):
     rodas = options.solver == "rodas5P"
     lu_t = "float" if options.lu_precision == "fp32" else "double"
     wide = wide_solve(options, n_vars)
+    closed = closed_inverse(options, n_vars)
+    if closed:
+        lu_t, wide = "double", False
     parts = [
         f"// generated problem source: {options.solver}, n_vars={n_vars}, n_params={n_params}, n_sens={n_sens}",
         f"#define MDX_NV {n_vars}",
@@ -468,7 +481,23 @@ def build_source(ode_fn, n_vars: int, n_params: int, options: KernelOptions):
     lu_size = 0
     sparse = None
     if rodas:
-        if options.sparsity is None and options.fast and n_vars <= DENSE_UNROLL_MAX:
+        if closed:
+            structure = dense_jacobian(n_vars)
+            lu_size = n_vars * n_vars
+            parts.append(f"#define MDX_LU_SIZE {lu_size}")
+            parts.append("#define MDX_IPIV 1")
+            parts.append("#define MDX_SCALED_SYSTEM 1")
+            parts.append('#include "mdx_dense_lu.cuh"')
+            parts.append(
+                "template <class LU, class IP> __device__ __forceinline__ void mdx_factorize(LU& lu, IP&) "
+                "{ mdx::closed_inverse<MDX_NV>(lu); }\n"
+                "template <class LU, class IP, class R> __device__ __forceinline__ void mdx_solve(const LU& lu, const IP&, R& rhs) "
+                "{ mdx::inverse_solve<MDX_NV, false>(lu, rhs); }\n"
+                "template <class LU, class IP, class R> __device__ __forceinline__ void mdx_solve_t(const LU& lu, const IP&, R& rhs) "
+                "{ mdx::inverse_solve<MDX_NV, true>(lu, rhs); }\n"
+                "__device__ __forceinline__ int mdx_diag_slot(int d) { return d * MDX_NV + d; }"
+            )
+        elif options.sparsity is None and options.fast and n_vars <= DENSE_UNROLL_MAX:
             structure = dense_jacobian(n_vars)
             lu_size = n_vars * n_vars
             parts.append(f"#define MDX_LU_SIZE {lu_size}")

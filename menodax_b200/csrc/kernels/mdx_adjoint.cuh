@@ -71,8 +71,7 @@ __device__ __forceinline__ void recompute(double t, double h, const double (&y)[
   SLU& lu = lus;
 #endif
   mdx_neg_jac(y, t, p, lu, dT);
-#pragma unroll
-  for (int d = 0; d < MDX_NV; ++d) lu[mdx_diag_slot(d)] += (T)dtgamma_inv;
+  shift_matrix(lu, h, dtgamma_inv);
   mdx_factorize(lu, ipiv);
 #if MDX_WIDE_SOLVE
   widen_factors(lu, lus);
@@ -104,7 +103,14 @@ __device__ __forceinline__ void recompute(double t, double h, const double (&y)[
 #pragma unroll
     for (int j = 0; j < MDX_NV; ++j) {
       double value;
-      if (s == 0) {
+      if (MDX_SCALED_SYSTEM) {
+        double f = work[j];
+        if (coef_d(s) != 0.0 && !MDX_AUTONOMOUS) f += h * coef_d(s) * dT[j];
+        double acc = 0.0;
+#pragma unroll
+        for (int m = 0; m < s; ++m) acc += GAMMA * coef_c(s, m) * (double)k[m][j];
+        value = acc + h * GAMMA * f;
+      } else if (s == 0) {
         value = MDX_AUTONOMOUS ? work[j] : work[j] + h * coef_d(0) * dT[j];
       } else {
         double acc = coef_c(s, 0) * (double)k[0][j];
@@ -206,8 +212,9 @@ __device__ __forceinline__ void reverse_step(const MdxGradArgs& a, int traj, dou
     mdx_solve_t(lu, ipiv, rb_t);
     double rbar[MDX_NV];
 #pragma unroll
-    for (int j = 0; j < MDX_NV; ++j) rbar[j] = (double)rb_t[j];
-    // k_s = W^-1 r_s with W = I/(h gamma) - J(y, p): J-bar = rbar k_s^T.
+    for (int j = 0; j < MDX_NV; ++j) rbar[j] = MDX_SCALED_SYSTEM ? h * GAMMA * (double)rb_t[j] : (double)rb_t[j];
+    // k_s = W^-1 r_s with W = I/(h gamma) - J(y, p) (a scaled system's M is
+    // h gamma W): J-bar = rbar k_s^T.
     double kd[MDX_NV];
 #pragma unroll
     for (int j = 0; j < MDX_NV; ++j) kd[j] = (double)k[s][j];

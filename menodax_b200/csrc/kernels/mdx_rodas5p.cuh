@@ -47,6 +47,12 @@ typedef MDX_LU_T lu_t;
 #define MDX_WIDE_SOLVE 0
 #endif
 typedef MDX_SOLVE_T sol_t;
+// Builds that invert their matrix in closed form solve the step's systems times
+// h gamma: (I - h gamma J) k = h gamma f + gamma sum C k.  The matrix then waits for
+// no reciprocal of h, a hundred dependent cycles at the head of every step.
+#ifndef MDX_SCALED_SYSTEM
+#define MDX_SCALED_SYSTEM 0
+#endif
 // Stage increments: small systems keep them in double registers (the rounded
 // values, or the wide solve's own), larger ones in the LU type unless the
 // solve is wide.
@@ -130,6 +136,35 @@ __device__ __forceinline__ bool running(const State& st, const MdxSolveArgs& a) 
   return st.save_idx < a.n_save && st.t < st.tf_local && st.n_steps < a.max_steps;
 }
 
+// h gamma f + gamma sum_m C_sm k_m of component j.
+template <int S, class K>
+__device__ __forceinline__ double scaled_rhs(double f, const K& k, int j, double h_gamma) {
+  if constexpr (S == 0) {
+    return h_gamma * f;
+  } else {
+    double acc = GAMMA * coef_c(S, 0) * (double)k[0][j];
+#pragma unroll
+    for (int m = 1; m < S; ++m) acc += GAMMA * coef_c(S, m) * (double)k[m][j];
+    return acc + h_gamma * f;
+  }
+}
+
+// M from -J: I/(h gamma) - J, or (MDX_SCALED_SYSTEM) I - h gamma J.
+template <class LU>
+__device__ __forceinline__ void shift_matrix(LU& lu, double h, double dtgamma_inv) {
+#if MDX_SCALED_SYSTEM
+  (void)dtgamma_inv;
+#pragma unroll
+  for (int i = 0; i < MDX_LU_SIZE; ++i) lu[i] *= h * GAMMA;
+#pragma unroll
+  for (int d = 0; d < MDX_NV; ++d) lu[mdx_diag_slot(d)] += 1.0;
+#else
+  (void)h;
+#pragma unroll
+  for (int d = 0; d < MDX_NV; ++d) lu[mdx_diag_slot(d)] += (lu_t)dtgamma_inv;
+#endif
+}
+
 // One Rosenbrock stage: its right-hand side from the tableau row, then the
 // solve against the step's factorisation.  State rows go to the solver's
 // buffer; with forward sensitivities the sensitivity rows wait in `work` until
@@ -141,7 +176,11 @@ __device__ __forceinline__ void stage(const LU& lu, const IP& ipiv, RB& rhs, K& 
 #pragma unroll
   for (int j = 0; j < MDX_NS; ++j) {
     double value;
-    if constexpr (S == 0) {
+    if constexpr (MDX_SCALED_SYSTEM) {
+      double f = work[j];
+      if constexpr (coef_d(S) != 0.0 && !MDX_AUTONOMOUS) f += dt_use * coef_d(S) * dT[j];
+      value = scaled_rhs<S>(f, k, j, dt_use * GAMMA);
+    } else if constexpr (S == 0) {
       if constexpr (MDX_AUTONOMOUS) value = work[j];
       else value = work[j] + dt_use * coef_d(0) * dT[j];
     } else {
@@ -214,8 +253,7 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a) {
   int ipiv[MDX_IPIV];
   double dT[MDX_NS];
   mdx_neg_jac(st.y, t, st.p, lu, dT);
-#pragma unroll
-  for (int d = 0; d < MDX_NV; ++d) lu[mdx_diag_slot(d)] += (lu_t)dtgamma_inv;
+  shift_matrix(lu, dt_use, dtgamma_inv);
   mdx_factorize(lu, ipiv);
 #if MDX_WIDE_SOLVE
   sol_t lus[MDX_LU_SIZE];

@@ -93,3 +93,36 @@ def test_kept_pivots_solve_to_the_same_bits(lib, t, n):
             run(_p(a), _p(b), _p(x), transposed, 1)
             run(_p(a), _p(b), _p(y), transposed, 0)
             np.testing.assert_array_equal(x, y)
+
+
+CLOSED = """
+#include "mdx_dense_lu.cuh"
+#define CLOSED(N) extern "C" void closed##N(const double* a, const double* b, double* x, double* xt) { \\
+  double m[N * N], r[N], rt[N]; for (int i = 0; i < N * N; ++i) m[i] = a[i]; for (int i = 0; i < N; ++i) r[i] = rt[i] = b[i]; \\
+  mdx::closed_inverse<N>(m); mdx::inverse_solve<N, false>(m, r); mdx::inverse_solve<N, true>(m, rt); \\
+  for (int i = 0; i < N; ++i) { x[i] = r[i]; xt[i] = rt[i]; } }
+CLOSED(1) CLOSED(2) CLOSED(3)
+"""
+
+
+@pytest.mark.parametrize("n", [1, 2, 3])
+def test_closed_inverse(tmp_path, n):
+    """Cofactors against NumPy: each entry is a few products, so the inverse is off by at
+    most about 8 n roundings times the condition number; a determinant past the range of a
+    double gives NaN, not the zero that would pass an error test."""
+    (tmp_path / "c.cpp").write_text(PRELUDE + CLOSED)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", f"-I{KERNEL_DIR}", str(tmp_path / "c.cpp"),
+                    "-o", str(tmp_path / "c.so")], check=True)
+    run = getattr(ctypes.CDLL(str(tmp_path / "c.so")), f"closed{n}")
+    rng = np.random.default_rng(n)
+    x, xt = np.empty(n), np.empty(n)
+    for _ in range(300):
+        a = rng.normal(size=(n, n)) * np.exp(rng.uniform(-12, 12, (n, 1)))
+        b = rng.normal(size=n)
+        run(_p(a), _p(b), _p(x), _p(xt))
+        inv = np.linalg.inv(a)
+        bound = 16 * n * 2.0 ** -53 * np.linalg.cond(a) * np.linalg.norm(inv) * np.linalg.norm(b)
+        assert np.linalg.norm(x - np.linalg.solve(a, b)) <= bound
+        assert np.linalg.norm(xt - np.linalg.solve(a.T, b)) <= bound
+    run(_p(np.eye(n) * 1e200 if n > 1 else np.array([[np.inf]])), _p(np.ones(n)), _p(x), _p(xt))
+    assert np.isnan(x).all()
