@@ -74,6 +74,7 @@ struct State {
   double y[MDX_NS];
   double p[MDX_NP > 0 ? MDX_NP : 1];
   double t, dt, err_prev, err_prev2, tf_local;
+  double next_save;  // times[save_idx]: read when the cursor moves, not on every step
   int save_idx, n_steps, accepted, rejected, traj;
 #if MDX_CHECKPOINT
   int n_ckpt;
@@ -108,6 +109,7 @@ __device__ __forceinline__ void init(State& st, const MdxSolveArgs& a, int traj)
   st.t = t0;
   st.dt = a.dt0 > 0.0 ? a.dt0 : (tf - t0) * 1e-6;
   st.save_idx = 1;
+  st.next_save = a.times[a.n_save > 1 ? 1 : 0];
   st.n_steps = 0;
   st.accepted = 0;
   st.rejected = 0;
@@ -336,11 +338,11 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a) {
     }
 #endif
     const double t_new = t + dt_use;
-    while (st.save_idx < a.n_save && save_reached(a.times[st.save_idx], t_new)) {
+    while (st.save_idx < a.n_save && save_reached(st.next_save, t_new)) {
 #if MDX_FAST
-      const double theta = (a.times[st.save_idx] - t) * inv_dt;
+      const double theta = (st.next_save - t) * inv_dt;
 #else
-      const double theta = div_by(a.times[st.save_idx] - t, dt_use, inv_dt);
+      const double theta = div_by(st.next_save - t, dt_use, inv_dt);
 #endif
       const double theta1 = 1.0 - theta;
 #if MDX_FAST
@@ -383,10 +385,11 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a) {
 #endif
       }
 #if MDX_HAS_HOOK
-      mdx_save_hook(st.save_idx, y_save, a.times[st.save_idx], st.p,
+      mdx_save_hook(st.save_idx, y_save, st.next_save, st.p,
                     a.hook_out + (size_t)st.traj * MDX_HOOK_SIZE);
 #endif
       ++st.save_idx;
+      if (st.save_idx < a.n_save) st.next_save = a.times[st.save_idx];
     }
 #pragma unroll
     for (int j = 0; j < MDX_NS; ++j) st.y[j] = u[j] + (double)k[7][j];
