@@ -226,7 +226,7 @@ def small_choice(ode_fn, n_vars, n_params, options, n) -> LaunchChoice | None:
     64.4 and 3.5 ms, on threads slower still).  Other systems of ``TEAM_MIN_VARS`` states or
     more take a team by the same rule: a thread's vectors no longer fit its registers, nor a
     dense matrix at all (256 trajectories: dense 32 states 94.6 ms on threads, 4.2 on
-    32-lane teams, 1.2 with the register inverse; sparse 64 states 0.75 on threads, 0.18 on
+    32-lane teams, 1.0 with the register inverse; sparse 64 states 0.75 on threads, 0.18 on
     32 lanes)."""
     lanes = cyclic_lanes(ode_fn, n_vars, n_params, options)
     if lanes:
@@ -242,19 +242,17 @@ def small_choice(ode_fn, n_vars, n_params, options, n) -> LaunchChoice | None:
         teams.append(t)
     if not teams:
         return None
-    if team_inverse_fits(n_vars, replace(options, team=teams[-1])):
-        # The inverse gains from lanes for longer: 32 states, 32 / 16 lanes, 1,500
-        # trajectories 2.04 / 2.56 ms, 4,097 5.0 / 5.4.
-        team = _spread(teams, n, 2 * SMALL_ENSEMBLE_LANES)
-    else:
-        team = _spread(teams, n)
+    # The register inverse gains from lanes at every such size: 32 states on 32 / 16 lanes,
+    # 256 trajectories 1.02 / 1.75 ms, 1,500 1.63 / 2.28, 4,097 3.79 / 4.77.
+    widest = max(teams)
+    team = widest if team_inverse_fits(n_vars, replace(options, team=widest)) else _spread(teams, n)
     return LaunchChoice(32, _native.MDX_LAUNCH_PLAIN, 0.0, team,
                         inverse=team_inverse_fits(n_vars, replace(options, team=team)))
 
 
-def _spread(lanes, n: int, most: int = SMALL_ENSEMBLE_LANES) -> int:
-    """The widest of ``lanes`` that keep ``n`` trajectories within ``most`` lanes in all."""
-    fitting = [t for t in lanes if t * n <= most]
+def _spread(lanes, n: int) -> int:
+    """The widest of ``lanes`` that keep ``n`` trajectories within ``SMALL_ENSEMBLE_LANES``."""
+    fitting = [t for t in lanes if t * n <= SMALL_ENSEMBLE_LANES]
     return max(fitting) if fitting else min(lanes)
 
 

@@ -213,62 +213,76 @@ __device__ __forceinline__ bool running(const State& st, const MdxSolveArgs& a) 
   return st.save_idx < a.n_save && st.t < st.tf_local && st.n_steps < a.max_steps;
 }
 
-// Component j of stage S's right-hand side.
-template <int S>
-__device__ __forceinline__ double stage_value(const Slice& s, int j, double dt_use, double inv_dt) {
-  if constexpr (S == 0) {
-#if MDX_TEAM_AUTONOMOUS
-    return s.f[j];
-#else
-    return s.f[j] + dt_use * coef_d(0) * s.dT[j];
-#endif
-  } else {
-    double acc = coef_c(S, 0) * (double)s.k[0][j];
-#pragma unroll
-    for (int m = 1; m < S; ++m) acc += coef_c(S, m) * (double)s.k[m][j];
-#if !MDX_TEAM_AUTONOMOUS
-    if constexpr (coef_d(S) != 0.0) return s.f[j] + dt_use * coef_d(S) * s.dT[j] + acc * inv_dt;
-#endif
-    return s.f[j] + acc * inv_dt;
-  }
-}
-
-// Stage S: its right-hand side (rounded to the LU type), then the solve, into k[S].
+// A lane's own components, and their stage increments: in registers beside a register
+// inverse, in the slice otherwise.
 #if MDX_TEAM_INVERSE
-template <int S>
-__device__ __forceinline__ void stage(Slice& s, const Inverse& m, const Lanes& L, double dt_use, double inv_dt) {
-  lu_t b[ROWS];
-#pragma unroll
-  for (int q = 0; q < ROWS; ++q) {
-    const int j = L.lane + q * MDX_TEAM;
-    b[q] = j < MDX_NV ? (lu_t)stage_value<S>(s, j, dt_use, inv_dt) : (lu_t)0;
-  }
-  apply(s, m, b, s.k[S], L);
-}
-#define MDX_TEAM_STAGE(S) stage<S>(s, inverse, L, dt_use, inv_dt)
+#define MDX_TEAM_OWN_PARAM , Inverse& inverse
+#define MDX_TEAM_OWN , inverse
+#define MDX_TEAM_EACH(j, q) \
+  _Pragma("unroll") for (int q = 0, j = L.lane; q < ROWS; ++q, j += MDX_TEAM) if (j < MDX_NV)
+#define MDX_TEAM_K(m, j, q) inverse.k[m][q]
 #else
-#define MDX_TEAM_STAGE(S) stage<S>(s, L, dt_use, inv_dt)
+#define MDX_TEAM_OWN_PARAM
+#define MDX_TEAM_OWN
+#define MDX_TEAM_EACH(j, q) for (int j = L.lane; j < MDX_NV; j += MDX_TEAM)
+#define MDX_TEAM_K(m, j, q) (double)s.k[m][j]
+#endif
+
+// Stage S's right-hand side into k[S] (rounded to the LU type), then the solve.
 template <int S>
-__device__ __forceinline__ void stage(Slice& s, const Lanes& L, double dt_use, double inv_dt) {
-  for (int j = L.lane; j < MDX_NV; j += MDX_TEAM) s.k[S][j] = (lu_t)stage_value<S>(s, j, dt_use, inv_dt);
+__device__ __forceinline__ void stage(Slice& s, const Lanes& L, double dt_use, double inv_dt MDX_TEAM_OWN_PARAM) {
+#if MDX_TEAM_INVERSE
+  lu_t b[ROWS];
+#endif
+  MDX_TEAM_EACH(j, q) {
+    double value;
+    if constexpr (S == 0) {
+#if MDX_TEAM_AUTONOMOUS
+      value = s.f[j];
+#else
+      value = s.f[j] + dt_use * coef_d(0) * s.dT[j];
+#endif
+    } else {
+      double acc = coef_c(S, 0) * MDX_TEAM_K(0, j, q);
+#pragma unroll
+      for (int m = 1; m < S; ++m) acc += coef_c(S, m) * MDX_TEAM_K(m, j, q);
+#if !MDX_TEAM_AUTONOMOUS
+      if constexpr (coef_d(S) != 0.0) {
+        value = s.f[j] + dt_use * coef_d(S) * s.dT[j] + acc * inv_dt;
+      } else {
+        value = s.f[j] + acc * inv_dt;
+      }
+#else
+      value = s.f[j] + acc * inv_dt;
+#endif
+    }
+#if MDX_TEAM_INVERSE
+    b[q] = (lu_t)value;
+  }
+  apply(s, inverse, b, s.k[S], L);
+  MDX_TEAM_EACH(j, q) inverse.k[S][q] = (double)s.k[S][j];
+#else
+    s.k[S][j] = (lu_t)value;
+  }
   __syncwarp(L.mask);
   solve(s, s.k[S], L);
-}
 #endif
+}
 
 template <int S>
-__device__ __forceinline__ void advance(Slice& s, const Lanes& L) {
-  for (int j = L.lane; j < MDX_NV; j += MDX_TEAM) {
-    double acc = coef_a(S, 0) * (double)s.k[0][j];
+__device__ __forceinline__ void advance(Slice& s, const Lanes& L MDX_TEAM_OWN_PARAM) {
+  MDX_TEAM_EACH(j, q) {
+    double acc = coef_a(S, 0) * MDX_TEAM_K(0, j, q);
 #pragma unroll
-    for (int m = 1; m <= S; ++m) acc += coef_a(S, m) * (double)s.k[m][j];
+    for (int m = 1; m <= S; ++m) acc += coef_a(S, m) * MDX_TEAM_K(m, j, q);
     s.u[j] = s.y[j] + acc;
   }
   __syncwarp(L.mask);
 }
 
-__device__ __forceinline__ void accumulate(Slice& s, const Lanes& L, int S) {
-  for (int j = L.lane; j < MDX_NV; j += MDX_TEAM) s.u[j] += (double)s.k[S][j];
+template <int S>
+__device__ __forceinline__ void accumulate(Slice& s, const Lanes& L MDX_TEAM_OWN_PARAM) {
+  MDX_TEAM_EACH(j, q) s.u[j] += MDX_TEAM_K(S, j, q);
   __syncwarp(L.mask);
 }
 
@@ -309,33 +323,33 @@ __device__ __forceinline__ void step(State& st, Slice& s, const Lanes& L, const 
 #endif
 
   rhs(s, L, s.y, t);
-  MDX_TEAM_STAGE(0);
-  advance<0>(s, L);
+  stage<0>(s, L, dt_use, inv_dt MDX_TEAM_OWN);
+  advance<0>(s, L MDX_TEAM_OWN);
   rhs(s, L, s.u, t + coef_ct(0) * dt_use);
-  MDX_TEAM_STAGE(1);
-  advance<1>(s, L);
+  stage<1>(s, L, dt_use, inv_dt MDX_TEAM_OWN);
+  advance<1>(s, L MDX_TEAM_OWN);
   rhs(s, L, s.u, t + coef_ct(1) * dt_use);
-  MDX_TEAM_STAGE(2);
-  advance<2>(s, L);
+  stage<2>(s, L, dt_use, inv_dt MDX_TEAM_OWN);
+  advance<2>(s, L MDX_TEAM_OWN);
   rhs(s, L, s.u, t + coef_ct(2) * dt_use);
-  MDX_TEAM_STAGE(3);
-  advance<3>(s, L);
+  stage<3>(s, L, dt_use, inv_dt MDX_TEAM_OWN);
+  advance<3>(s, L MDX_TEAM_OWN);
   rhs(s, L, s.u, t + coef_ct(3) * dt_use);
-  MDX_TEAM_STAGE(4);
-  advance<4>(s, L);
+  stage<4>(s, L, dt_use, inv_dt MDX_TEAM_OWN);
+  advance<4>(s, L MDX_TEAM_OWN);
   rhs(s, L, s.u, t_end);
-  MDX_TEAM_STAGE(5);
-  accumulate(s, L, 5);
+  stage<5>(s, L, dt_use, inv_dt MDX_TEAM_OWN);
+  accumulate<5>(s, L MDX_TEAM_OWN);
   rhs(s, L, s.u, t_end);
-  MDX_TEAM_STAGE(6);
-  accumulate(s, L, 6);
+  stage<6>(s, L, dt_use, inv_dt MDX_TEAM_OWN);
+  accumulate<6>(s, L MDX_TEAM_OWN);
   rhs(s, L, s.u, t_end);
-  MDX_TEAM_STAGE(7);
+  stage<7>(s, L, dt_use, inv_dt MDX_TEAM_OWN);
 
   // Weighted RMS of k8 (modax/rodas5P.py:903-911): scaled terms by component on
   // the owning lanes, then the sum of squares in component order on every lane.
-  for (int j = L.lane; j < MDX_NV; j += MDX_TEAM) {
-    const double k7 = (double)s.k[7][j];
+  MDX_TEAM_EACH(j, q) {
+    const double k7 = MDX_TEAM_K(7, j, q);
     const double y_new_j = s.u[j] + k7;
     const double scale = a.atol + a.rtol * pymax(fabs(s.y[j]), fabs(y_new_j));
 #if MDX_FAST
@@ -403,24 +417,24 @@ __device__ __forceinline__ void step(State& st, Slice& s, const Lanes& L, const 
 #pragma unroll
       for (int m = 0; m < 8; ++m) w[m] = coef_h(0, m) + theta * (coef_h(1, m) + theta * coef_h(2, m));
 #endif
-      for (int j = L.lane; j < MDX_NV; j += MDX_TEAM) {
+      MDX_TEAM_EACH(j, q) {
 #if MDX_FAST
-        double hsum = w[0] * (double)s.k[0][j];
+        double hsum = w[0] * MDX_TEAM_K(0, j, q);
 #pragma unroll
-        for (int m = 1; m < 8; ++m) hsum += w[m] * (double)s.k[m][j];
-        const double y_new_j = s.u[j] + (double)s.k[7][j];
+        for (int m = 1; m < 8; ++m) hsum += w[m] * MDX_TEAM_K(m, j, q);
+        const double y_new_j = s.u[j] + MDX_TEAM_K(7, j, q);
         const double val = theta1 * s.y[j] + theta * (y_new_j + theta1 * hsum);
 #else
-        double h1 = coef_h(0, 0) * (double)s.k[0][j];
-        double h2 = coef_h(1, 0) * (double)s.k[0][j];
-        double h3 = coef_h(2, 0) * (double)s.k[0][j];
+        double h1 = coef_h(0, 0) * MDX_TEAM_K(0, j, q);
+        double h2 = coef_h(1, 0) * MDX_TEAM_K(0, j, q);
+        double h3 = coef_h(2, 0) * MDX_TEAM_K(0, j, q);
 #pragma unroll
         for (int m = 1; m < 8; ++m) {
-          h1 += coef_h(0, m) * (double)s.k[m][j];
-          h2 += coef_h(1, m) * (double)s.k[m][j];
-          h3 += coef_h(2, m) * (double)s.k[m][j];
+          h1 += coef_h(0, m) * MDX_TEAM_K(m, j, q);
+          h2 += coef_h(1, m) * MDX_TEAM_K(m, j, q);
+          h3 += coef_h(2, m) * MDX_TEAM_K(m, j, q);
         }
-        const double y_new_j = s.u[j] + (double)s.k[7][j];
+        const double y_new_j = s.u[j] + MDX_TEAM_K(7, j, q);
         const double val = theta1 * s.y[j] + theta * (y_new_j + theta1 * (h1 + theta * (h2 + theta * h3)));
 #endif
 #if MDX_SAVE_HISTORY
@@ -440,7 +454,7 @@ __device__ __forceinline__ void step(State& st, Slice& s, const Lanes& L, const 
 #endif
       ++st.save_idx;
     }
-    for (int j = L.lane; j < MDX_NV; j += MDX_TEAM) s.y[j] = s.u[j] + (double)s.k[7][j];
+    MDX_TEAM_EACH(j, q) s.y[j] = s.u[j] + MDX_TEAM_K(7, j, q);
     st.t += dt_use;
     ++st.accepted;
   } else {

@@ -104,10 +104,10 @@ __device__ __forceinline__ void recompute(Slice& s, const Lanes& L, double t, do
   advance<4>(s, L);
   rhs(s, L, s.u, t_end);
   stage<5>(s, L, h, inv_dt);
-  accumulate(s, L, 5);
+  accumulate<5>(s, L);
   rhs(s, L, s.u, t_end);
   stage<6>(s, L, h, inv_dt);
-  accumulate(s, L, 6);
+  accumulate<6>(s, L);
   rhs(s, L, s.u, t_end);
   stage<7>(s, L, h, inv_dt);
 }

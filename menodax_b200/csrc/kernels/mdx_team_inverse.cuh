@@ -11,9 +11,9 @@
 // the 2/3 n^3 of a factorisation, at one shared-memory access per four of them
 // instead of 1.25 per one in mdx_team_lu.cuh).  The dense Brusselator on a B200, LU in
 // shared memory / inverse here, each at its best team: 32 states, 1 trajectory 3.7 /
-// 1.05 ms, 256 4.2 / 1.18, 4,097 7.6 / 4.7, 16,384 28.1 / 15.2; 16 states, 4,097 2.7 /
-// 1.36; 64 states, 4,097 44.6 / 21.2.  The LU stays for matrices whose rows do not fit
-// the registers (team_inverse_fits) and for the arithmetic it shares with the reference.
+// 0.92 ms, 256 4.2 / 1.02, 4,097 7.6 / 3.8, 16,384 28.1 / 12.8; 16 states, 4,097 2.7 /
+// 1.18; 64 states, 4,097 44.6 / 17.9.  The LU stays for matrices whose rows do not
+// fit the registers (team_inverse_fits) and for the reference's arithmetic.
 //
 // Rows stay where they are: `column[q]` is the column whose pivot row q was, so row
 // q of the inverse gives that component, and pivots are not applied until the end
@@ -32,13 +32,17 @@ struct Inverse {
   lu_t a[ROWS][MDX_NV];
   lu_t scale[ROWS];
   int column[ROWS];
+  double k[8][ROWS];  // the lane's own components of the stage increments, widened once
 };
 
 // Two vectors at the front of the matrix's shared memory, free once its rows are in
-// registers: 16-byte aligned, one ahead of the other's readers.
+// registers: 16-byte aligned, one ahead of the other's readers.  The offset is reckoned
+// in integers: a pointer rounded up by a cast is no longer known to point to shared
+// memory, and its loads, then generic ones, were what the inversion waited for.
 __device__ __forceinline__ lu_t* exchange(Slice& s, int which) {
-  const size_t at = ((size_t)s.lu + 15) & ~(size_t)15;
-  return reinterpret_cast<lu_t*>(at) + which * (PADDED + 4);
+  const unsigned at = (threadIdx.x / MDX_TEAM) * (unsigned)MDX_TEAM_SLICE_BYTES
+                      + (unsigned)((const char*)s.lu - (const char*)&s);
+  return s.lu + ((0u - at) & 15u) / (unsigned)sizeof(lu_t) + which * (PADDED + 4);
 }
 static_assert(4 * MDX_TEAM_LU_SIZE >= 16 + 8 * (PADDED + 4), "the matrix's memory holds both vectors");
 
@@ -61,8 +65,10 @@ __device__ __forceinline__ void invert(Slice& s, Inverse& m, const Lanes& L) {
     // The largest remaining entry, its row number in the low bits: magnitudes are
     // told apart to one part in 2^17.
     unsigned best = 0;
+    lu_t recip[ROWS];  // every row's, ready before the search has found the pivot
 #pragma unroll
     for (int q = 0; q < ROWS; ++q) {
+      recip[q] = fast_recip(m.a[q][0]);
       const unsigned key = (__float_as_uint(fabsf(m.a[q][0])) & ~63u) | (unsigned)(63 - (L.lane + q * MDX_TEAM));
       if (!used[q] && key > best) best = key;
     }
@@ -72,7 +78,7 @@ __device__ __forceinline__ void invert(Slice& s, Inverse& m, const Lanes& L) {
 #pragma unroll
     for (int q = 0; q < ROWS; ++q) {
       if (pivot == L.lane + q * MDX_TEAM) {
-        // The row as the next columns' order has it, then the pivot.
+        // The row as the next columns' order has it, then the pivot's reciprocal.
         Four* const out = reinterpret_cast<Four*>(x);
 #pragma unroll
         for (int j = 0; j < PADDED; j += 4) {
@@ -81,11 +87,11 @@ __device__ __forceinline__ void invert(Slice& s, Inverse& m, const Lanes& L) {
           for (int e = 0; e < 4; ++e) f.v[e] = m.a[q][j + e + 1 < MDX_NV ? j + e + 1 : 0];
           out[j / 4] = f;
         }
-        x[PADDED] = m.a[q][0];
+        x[PADDED] = recip[q];
       }
     }
     __syncwarp(L.mask);
-    const lu_t inv = fast_recip(x[PADDED]);
+    const lu_t inv = x[PADDED];
     lu_t f[ROWS], first[ROWS];
 #pragma unroll
     for (int q = 0; q < ROWS; ++q) {
@@ -130,9 +136,11 @@ __device__ __forceinline__ void apply(Slice& s, const Inverse& m, const lu_t (&b
   for (int q = 0; q < ROWS; ++q)
     if (L.lane + q * MDX_TEAM < MDX_NV) x[m.column[q]] = b[q];
   __syncwarp(L.mask);
-  lu_t acc[ROWS];
+  lu_t acc[ROWS][4];  // four chains: a solve waits for a quarter of its row's multiply-adds
 #pragma unroll
-  for (int q = 0; q < ROWS; ++q) acc[q] = (lu_t)0;
+  for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[q][e] = (lu_t)0;
   const Four* const in = reinterpret_cast<const Four*>(x);
 #pragma unroll
   for (int j = 0; j < PADDED; j += 4) {
@@ -141,13 +149,13 @@ __device__ __forceinline__ void apply(Slice& s, const Inverse& m, const lu_t (&b
     for (int e = 0; e < 4; ++e) {
       if (j + e < MDX_NV) {
 #pragma unroll
-        for (int q = 0; q < ROWS; ++q) acc[q] += m.a[q][j + e] * p.v[e];
+        for (int q = 0; q < ROWS; ++q) acc[q][e] += m.a[q][j + e] * p.v[e];
       }
     }
   }
 #pragma unroll
   for (int q = 0; q < ROWS; ++q)
-    if (L.lane + q * MDX_TEAM < MDX_NV) out[m.column[q]] = acc[q];
+    if (L.lane + q * MDX_TEAM < MDX_NV) out[m.column[q]] = (acc[q][0] + acc[q][1]) + (acc[q][2] + acc[q][3]);
   __syncwarp(L.mask);
 }
 
