@@ -101,11 +101,22 @@ def stream_key(device):
 
 
 def to_device(t, device):
+    """``t`` on ``device``, contiguous.
+
+    A host tensor is copied without waiting for the stream: the driver has read pageable
+    memory by the time an asynchronous copy from it returns, so the caller may change or free it
+    at once (page-locked memory it reads later, as it did before).  A waiting copy of the save
+    times alone (160 bytes) made each solve wait for the one before: 100 us of a 200 us call
+    on a B200.  During a stream capture the copy waits, which the capture refuses, rather than
+    become a node that reads host memory at replay."""
     if t is None:
         return None
     if t.device == device and t.is_contiguous():
         return t
-    return t.to(device=device, non_blocking=t.is_pinned() if not t.is_cuda else False).contiguous()
+    if t.is_cuda or device.type != "cuda":
+        return t.to(device=device).contiguous()
+    waits = not t.is_pinned() and torch.cuda.is_current_stream_capturing()
+    return t.contiguous().to(device=device, non_blocking=not waits)
 
 
 class Workspace:

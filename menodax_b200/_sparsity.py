@@ -78,7 +78,9 @@ def normalize_sparsity(sparsity, n_vars: int) -> tuple[tuple[int, ...], ...]:
         )
     mask = np.zeros((n_vars, n_vars), dtype=bool)
     mask[rows, cols] = True
-    return tuple(tuple(int(c) for c in np.flatnonzero(row)) for row in mask)
+    columns = np.nonzero(mask)[1].tolist()  # row by row
+    ends = np.cumsum(mask.sum(axis=1)).tolist()
+    return tuple(tuple(columns[start:end]) for start, end in zip([0, *ends], ends))
 
 
 @dataclass(frozen=True)

@@ -281,6 +281,20 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
     winner runs as a persistent launch, which refills lanes as the uneven
     trajectories finish."""
     n = y0.shape[0]
+    # A call that was tuned before needs none of the candidates.
+    call = (ode_fn, n_vars, n_params, options, n, max_steps, y0.device, tune_block, tune_team, tune_shared, tune_registers)
+    with _lock:
+        found = _cache.get(call)
+    if found is None:
+        found = _tuned(call, y0=y0, times=times, params=params, weights=weights, dt0=dt0, rtol=rtol, atol=atol,
+                       n_save_hist=n_save_hist)
+        with _lock:
+            _cache[call] = found
+    return found
+
+
+def _tuned(call, *, y0, times, params, weights, dt0, rtol, atol, n_save_hist):
+    ode_fn, n_vars, n_params, options, n, max_steps, _, tune_block, tune_team, tune_shared, tune_registers = call
     if options.team:
         blocks, teams = (), ((options.team, options.threads_per_block),)
     else:
