@@ -214,6 +214,14 @@ int mdx_grad(mdx_plan* plan, const mdx_grad_desc* desc, void* stream);
 int mdx_order_workspace_size(size_t* bytes);
 int mdx_order_longest_first(const int* steps, int n, int* order, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The contraction a forward-sensitivity gradient ends in: for every trajectory i and
+ * direction k, the sum over saves s and states r of cotangent[i, s, r] times the joint
+ * history's d y_r(t_s) / d theta_k.  `joint` is (n_traj, n_save, n_vars * (1 + n_sens)) as a joint
+ * solve writes it, `cotangent` (n_traj, n_save, n_vars).  Directions below n_first go to `first`
+ * (n_traj, n_first), the others to `rest` (n_traj, n_sens - n_first). */
+int mdx_sens_contract(const double* joint, const double* cotangent, int n_traj, int n_save, int n_vars,
+                      int n_sens, int n_first, double* first, double* rest, void* stream);
+
 /* Measured FMA throughput of the current device's CUDA cores, in FLOP/s
  * (an FMA counts two): the roofline denominator of the ensemble kernels, which
  * are bound by FP64/FP32 issue rather than HBM or the tensor cores.  No

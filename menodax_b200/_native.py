@@ -44,6 +44,7 @@ EXPORTED = (
     "mdx_occupancy", "mdx_solve", "mdx_grad", "mdx_last_error", "mdx_version",
     "mdx_measure_fma_peak", "mdx_solve_persistent_noalloc", "mdx_checkpoint_size",
     "mdx_order_workspace_size", "mdx_order_longest_first",
+    "mdx_sens_contract",
 )
 
 
@@ -92,7 +93,7 @@ class GradDesc(ctypes.Structure):
 
 def _library_sources():
     return [CSRC / "mdx_runtime.cpp", CSRC / "mdx_peak.cu", CSRC / "mdx_noalloc.cu",
-            CSRC / "mdx_order.cu", CSRC / "mdx_internal.h", KERNEL_DIR / "mdx_args.h", INCLUDE_DIR / "menodax.h"]
+            CSRC / "mdx_order.cu", CSRC / "mdx_contract.cu", CSRC / "mdx_internal.h", KERNEL_DIR / "mdx_args.h", INCLUDE_DIR / "menodax.h"]
 
 
 def build_library(force: bool = False) -> Path:
@@ -106,6 +107,7 @@ def build_library(force: bool = False) -> Path:
         str(CUDA_HOME / "bin" / "nvcc"), "-O2", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC",
         "-Xcompiler", "-Wall", f"-I{CUDA_HOME / 'include'}", str(CSRC / "mdx_runtime.cpp"), str(CSRC / "mdx_peak.cu"),
         str(CSRC / "mdx_noalloc.cu"), str(CSRC / "mdx_order.cu"),
+        str(CSRC / "mdx_contract.cu"),
         "-o", str(LIB_PATH), f"-L{CUDA_HOME / 'lib64'}", "-lnvrtc", "-ldl",
         f"-Xlinker=-rpath,{CUDA_HOME / 'lib64'}",
     ]
@@ -151,6 +153,7 @@ def lib():
         L.mdx_order_workspace_size.argtypes = [ctypes.POINTER(ctypes.c_size_t)]
         L.mdx_order_longest_first.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,
                                               ctypes.c_size_t, ctypes.c_void_p]
+        L.mdx_sens_contract.argtypes = ([ctypes.c_void_p] * 2 + [ctypes.c_int] * 5 + [ctypes.c_void_p] * 3)
         L.mdx_measure_fma_peak.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
         _lib = L
         return _lib
@@ -173,6 +176,13 @@ def order_longest_first(steps: int, n: int, order: int, workspace: int, nbytes: 
     """``mdx_order_longest_first`` on device addresses, in the current context."""
     check(lib().mdx_order_longest_first(steps, n, order, workspace, nbytes, ctypes.c_void_p(stream)),
           "mdx_order_longest_first")
+
+
+def sens_contract(joint: int, cotangent: int, n_traj: int, n_save: int, n_vars: int, n_sens: int, n_first: int,
+                  first: int | None, rest: int | None, stream: int) -> None:
+    """``mdx_sens_contract`` on device addresses, in the current context."""
+    check(lib().mdx_sens_contract(joint, cotangent, n_traj, n_save, n_vars, n_sens, n_first, first, rest,
+                                  ctypes.c_void_p(stream)), "mdx_sens_contract")
 
 
 def last_error() -> str:

@@ -36,7 +36,7 @@ from dataclasses import replace
 import torch
 
 from menodax_b200 import _native, autotune
-from menodax_b200._ensemble import initial_step, launch, pick_device, solver_stats, stream_key
+from menodax_b200._ensemble import initial_step, launch, pick_device, solver_stats, stream_key, to_device
 from menodax_b200._problem import get_problem
 
 # Checkpoint capacity (accepted steps per trajectory) and stride last used per
@@ -88,6 +88,8 @@ def checkpoint_bytes(n_traj, n_vars, capacity, stride):
 
 def choose_stride(n_traj, n_vars, capacity, device):
     free, _ = torch.cuda.mem_get_info(device)
+    if checkpoint_bytes(n_traj, n_vars, capacity, CKPT_STRIDES[0]) <= MEMORY_FRACTION * free:
+        return CKPT_STRIDES[0]
     # Memory torch's caching allocator holds for no live tensor -- the previous
     # call's checkpoint buffer, typically -- is free for this one too; leaving it
     # out would pick a coarser stride on every call after the first, and a
@@ -261,7 +263,7 @@ class _EnsembleSolve(torch.autograd.Function):
         d.status = status.data_ptr()
         stream = torch.cuda.current_stream(params.device).cuda_stream
         plan = None
-        if not problem.options.team and REVERSE_CHUNK is None:
+        if REVERSE_SPLIT is not None and not problem.options.team and REVERSE_CHUNK is None:
             plan = split_plan(ckpt_count.cpu(), ctx.capacity, int(problem.options.ckpt_stride), problem.n_vars)
         if plan is not None:
             tasks, n_slots, combine = plan
@@ -324,35 +326,58 @@ class _Problems:
         return get_problem(*self.args, opts)
 
 
+def _plain(*tensors) -> bool:
+    """Whether a backward's tensors are ordinary contiguous CUDA doubles outside any
+    transform: what a native kernel may take.  Double backward, batched gradients, tracing and
+    saved-tensor hooks that changed the layout keep to torch operations."""
+    return not torch.is_grad_enabled() and all(
+        type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float64 and t.is_contiguous()
+        and torch._C._has_storage(t) and not torch._C._functorch.is_functorch_wrapped_tensor(t) for t in tensors)
+
+
 class _SensitivitySolve(torch.autograd.Function):
     """Forward sensitivities: the joint solve forward, ``S^T g`` backward."""
 
     @staticmethod
     def forward(ctx, y0, params, run):
-        state, sens, counters = run(y0.detach(), params.detach())
-        ctx.save_for_backward(sens)
+        hist, counters = run(y0.detach(), params.detach())
+        ctx.save_for_backward(hist)
+        ctx.n_vars = y0.shape[1]
         ctx.n_params = params.shape[1]
         ctx.wrt_y0 = run.wrt_y0
         ctx.columns = run.columns
         ctx.mark_non_differentiable(counters)
-        return state, counters
+        return hist[:, :, :ctx.n_vars].contiguous(), counters
 
     @staticmethod
     def backward(ctx, grad_state, _grad_counters):
-        (sens,) = ctx.saved_tensors
-        n, _, n_vars, _ = sens.shape
-        grad_y0 = grad_p = None
-        offset = 0
-        g = grad_state if grad_state is not None else torch.zeros(sens.shape[:3], dtype=sens.dtype,
-                                                                  device=sens.device)
-        if ctx.wrt_y0:
-            grad_y0 = torch.einsum("nsi,nsij->nj", g, sens[..., :n_vars])
-            offset = n_vars
+        (hist,) = ctx.saved_tensors
+        (n, n_save, width), n_vars = hist.shape, ctx.n_vars
+        n_sens = width // n_vars - 1
+        n_first = n_vars if ctx.wrt_y0 else 0
+        g = grad_state if grad_state is not None else torch.zeros((n, n_save, n_vars), dtype=hist.dtype,
+                                                                  device=hist.device)
+        if _plain(hist, g.contiguous()):
+            g = g.contiguous()
+            grad_y0 = torch.empty((n, n_first), dtype=hist.dtype, device=hist.device)
+            grad_cols = torch.empty((n, n_sens - n_first), dtype=hist.dtype, device=hist.device)
+            with torch.cuda.device(hist.device):
+                _native.sens_contract(hist.data_ptr(), g.data_ptr(), n, n_save, n_vars, n_sens, n_first,
+                                      grad_y0.data_ptr(), grad_cols.data_ptr(),
+                                      torch.cuda.current_stream(hist.device).cuda_stream)
+        else:
+            sens = hist[:, :, n_vars:].reshape(n, n_save, n_sens, n_vars)
+            grad_y0 = torch.einsum("nsi,nsji->nj", g, sens[:, :, :n_first])
+            grad_cols = torch.einsum("nsi,nski->nk", g, sens[:, :, n_first:])
+        grad_p = None
         if ctx.columns is not None:
-            grad_p = torch.zeros((n, ctx.n_params), dtype=sens.dtype, device=sens.device)
-            if ctx.columns:
-                grad_p[:, list(ctx.columns)] = torch.einsum("nsi,nsik->nk", g, sens[..., offset:])
-        return grad_y0, grad_p, None
+            if tuple(ctx.columns) == tuple(range(ctx.n_params)):
+                grad_p = grad_cols
+            else:
+                grad_p = torch.zeros((n, ctx.n_params), dtype=hist.dtype, device=hist.device)
+                if ctx.columns:
+                    grad_p[:, list(ctx.columns)] = grad_cols
+        return grad_y0 if ctx.wrt_y0 else None, grad_p, None
 
 
 class _JointRun:
@@ -366,13 +391,11 @@ class _JointRun:
     def __call__(self, y0, params):
         from menodax_b200 import sensitivity
 
-        state, sens, stats = sensitivity.solve(
+        hist, counters, _ = sensitivity.solve_joint(
             self.solver, self.ode_fn, y0, self.times, params, wrt_y0=self.wrt_y0,
             wrt_params=self.columns is not None and len(self.columns) > 0,
-            sens_error_control=True, sens_param_columns=self.columns or None,
-            return_stats=True, **self.kw)
-        counters = torch.stack([stats["accepted_steps"], stats["rejected_steps"], stats["loop_steps"]])
-        return state.contiguous(), sens.contiguous(), counters
+            sens_error_control=True, sens_param_columns=self.columns or None, **self.kw)
+        return hist, counters[:3]
 
 
 def _forward_sensitivity_grad(options, ode_fn, y0_t, p_t, times, *, rtol, atol, first_step, max_steps,
@@ -418,10 +441,9 @@ def solve_with_grad(ode_fn, y0, t_span, params, options, *, rtol, atol, first_st
     if p_t.ndim == 1:
         p_t = p_t.unsqueeze(0).expand(n, -1)
     n_vars, n_params = y0_t.shape[1], p_t.shape[1]
-    if isinstance(t_span, torch.Tensor):
-        times = t_span.detach().to(device=device, dtype=torch.float64).contiguous()
-    else:
-        times = torch.as_tensor(t_span, dtype=torch.float64, device=device).contiguous()
+    # Kept on the host too: the hints' keys read them without waiting for the device.
+    times_h = torch.as_tensor(t_span, dtype=torch.float64).detach()
+    times = to_device(times_h, device)
     if sens_param_columns is not None:
         cols = [int(c) for c in sens_param_columns]
         if len(set(cols)) != len(cols):
@@ -430,7 +452,7 @@ def solve_with_grad(ode_fn, y0, t_span, params, options, *, rtol, atol, first_st
         if bad:
             raise ValueError(f"param_columns {bad} lie outside the {n_params} parameter columns")
     if sens_error_control:
-        return _forward_sensitivity_grad(options, ode_fn, y0_t, p_t, times, rtol=rtol, atol=atol,
+        return _forward_sensitivity_grad(options, ode_fn, y0_t, p_t, times_h, rtol=rtol, atol=atol,
                                          first_step=first_step, max_steps=max_steps,
                                          return_stats=return_stats, sens_param_columns=sens_param_columns)
     if sens_param_columns is not None and p_t.requires_grad:
@@ -438,7 +460,7 @@ def solve_with_grad(ode_fn, y0, t_span, params, options, *, rtol, atol, first_st
         keep[list(int(c) for c in sens_param_columns)] = 1.0
         p_t = _ColumnMask.apply(p_t, keep)
     problems = _Problems(ode_fn, n_vars, n_params, replace(options, runtime_weights=False))
-    key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol),
+    key = (ode_fn, n_vars, n_params, options, n, tuple(times_h.tolist()), float(rtol), float(atol),
            stream_key(device))
     hist, counters = _EnsembleSolve.apply(y0_t, p_t, times, problems, initial_step(first_step), rtol,
                                           atol, max_steps, key)

@@ -118,6 +118,22 @@ def solve(solver, ode_fn, y0, t_span, params, *, wrt_y0=True, wrt_params=True,
     ``solver`` is ``"tsit5"`` or ``"rodas5P"``.  ``S[n, s, r, k]`` is
     ``d y_r(t_s) / d theta_k`` for direction ``k`` (y0 directions first, then the
     parameter columns)."""
+    hist, counters, spec = solve_joint(
+        solver, ode_fn, y0, t_span, params, wrt_y0=wrt_y0, wrt_params=wrt_params, sens_error_control=sens_error_control,
+        sens_param_columns=sens_param_columns, rtol=rtol, atol=atol, first_step=first_step, max_steps=max_steps,
+        lu_precision=lu_precision, sparsity=sparsity, ordering=ordering, pcoeff=pcoeff, icoeff=icoeff, dcoeff=dcoeff)
+    state, sens = split_augmented(hist, spec)
+    if return_stats:
+        from menodax_b200._ensemble import solver_stats
+
+        return state, sens, solver_stats(counters[0], counters[1], counters[2])
+    return state, sens
+
+
+def solve_joint(solver, ode_fn, y0, t_span, params, *, wrt_y0, wrt_params, sens_error_control, sens_param_columns, rtol,
+                atol, first_step, max_steps, lu_precision="fp64", sparsity=None, ordering="amd", pcoeff=0.0,
+                icoeff=1.0, dcoeff=0.0):
+    """The joint solve itself: its history ``(n, S, n_aug)``, counters and ``SensitivitySpec``."""
     if solver not in ("tsit5", "rodas5P"):
         raise ValueError(f"solver must be 'tsit5' or 'rodas5P'; got {solver!r}")
     y0_t, p_t, n, n_vars = normalize_y0_params(y0, params)
@@ -139,16 +155,17 @@ def solve(solver, ode_fn, y0, t_span, params, *, wrt_y0=True, wrt_params=True,
     problem = get_problem(ode_fn, n_vars, n_params, options)
     z0 = augmented_y0(to_device(y0_t.detach(), device), spec)
     if isinstance(t_span, torch.Tensor):
-        times = t_span.detach().to(device=device, dtype=torch.float64).contiguous()
+        times_h = t_span.detach().to(torch.float64)
     else:
-        times = torch.as_tensor(np.asarray(t_span, dtype=np.float64), device=device).contiguous()
+        times_h = torch.as_tensor(np.asarray(t_span, dtype=np.float64))
+    times = to_device(times_h, device)
     # The persistent refill launch, trajectories longest first by the previous
     # call's step counts for the same problem: the joint solves are long and
     # uneven, and the order only moves when each trajectory runs (the 2-state
     # stiff Van der Pol gradients of 65,536 trajectories: 324 ms plain, 207 ms
     # persistent, 163 ms persistent longest first; the same gradients bit for
     # bit).
-    key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol),
+    key = (ode_fn, n_vars, n_params, options, n, tuple(times_h.tolist()), float(rtol), float(atol),
            stream_key(device))
     order = _order_hint.get(key)
     if order is not None and (order.device != device or order.numel() != n):
@@ -162,12 +179,7 @@ def solve(solver, ode_fn, y0, t_span, params, *, wrt_y0=True, wrt_params=True,
     _order_hint[key] = autotune.longest_first(counters[0])
     while len(_order_hint) > ORDER_HINT_PROBLEMS:
         _order_hint.pop(next(iter(_order_hint)))
-    state, sens = split_augmented(hist, spec)
-    if return_stats:
-        from menodax_b200._ensemble import solver_stats
-
-        return state, sens, solver_stats(counters[0], counters[1], counters[2])
-    return state, sens
+    return hist, counters, spec
 
 
 def jvp(solver, ode_fn, y0, t_span, params, dy0=None, dparams=None, **kw):
