@@ -24,12 +24,11 @@ namespace mdx {
 namespace adjoint {
 
 __device__ __forceinline__ double ckpt_h(const MdxGradArgs& a, int m, int traj) {
-  return a.ckpt[(size_t)m * (size_t)a.n_traj + (size_t)traj];
+  return ckpt_record(a.ckpt, a.ckpt_capacity, m / MDX_CKPT_SEG, traj)[MDX_NV + 1 + m % MDX_CKPT_SEG];
 }
 
 __device__ __forceinline__ const double* ckpt_seg_state(const MdxGradArgs& a, int seg, int traj) {
-  return a.ckpt + (size_t)a.ckpt_capacity * (size_t)a.n_traj +
-         ((size_t)seg * (size_t)a.n_traj + (size_t)traj) * (size_t)(MDX_NV + 1);
+  return ckpt_record(a.ckpt, a.ckpt_capacity, seg, traj);
 }
 
 // The highest save index whose time a step ending at `t_end` reaches, searching
@@ -408,7 +407,7 @@ __device__ __forceinline__ void load_segment(const MdxGradArgs& a, int seg, int 
   const int m0 = seg * MDX_CKPT_SEG;
 #pragma unroll
   for (int k = 0; k < MDX_CKPT_SEG; ++k)
-    if (m0 + k < steps) d.h[k] = __ldg(a.ckpt + (size_t)(m0 + k) * (size_t)a.n_traj + (size_t)traj);
+    if (m0 + k < steps) d.h[k] = __ldg(rec + MDX_NV + 1 + k);
 #endif
 }
 

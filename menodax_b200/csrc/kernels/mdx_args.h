@@ -28,8 +28,8 @@ typedef struct MdxSolveArgs {
   double* hook_out;        /* (N, hook_size) or NULL */
   int* work_counter;       /* persistent kernels: queue head, zeroed before launch */
   const int* order;        /* persistent kernels: optional visiting order (N,) */
-  double* ckpt;            /* adjoint forward pass: step sizes (capacity, N), then segment
-                              start states (ceil(capacity / MDX_CKPT_SEG), N, n_vars + 1) */
+  double* ckpt;            /* adjoint forward pass: per trajectory a record (t, y, step sizes) for
+                              every MDX_CKPT_SEG steps (mdx_common.cuh) */
   int* ckpt_count;         /* adjoint forward pass: accepted steps recorded per trajectory */
   long long ckpt_capacity; /* steps per trajectory the checkpoint buffer holds */
   double* hist_host;       /* page-locked host copy of hist (device-mapped address), or NULL */
@@ -53,7 +53,7 @@ typedef struct MdxGradArgs {
   int* status;             /* may be NULL */
   const int* order;        /* may be NULL: thread i takes trajectory order[i] */
   long long ckpt_capacity;
-  int n_traj;              /* trajectories in the buffers (their stride) */
+  int n_traj;              /* trajectories in the buffers */
   int n_save;
   int n_run;               /* threads of this launch: order[0..n_run), or tasks[0..n_run) */
   const int* tasks;        /* split reverse: (n_run, 5) traj, first segment, end segment, kind, slot */

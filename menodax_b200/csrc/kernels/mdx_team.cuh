@@ -387,9 +387,9 @@ __device__ __forceinline__ void step(State& st, Slice& s, const Lanes& L, const 
     // The thread kernel's checkpoint layout (mdx_common.cuh::ckpt_write): the
     // step size, and every MDX_CKPT_SEG-th step's start (t, y), y by component.
     if (st.n_ckpt < a.ckpt_capacity) {
-      if (L.lane == 0) a.ckpt[(size_t)st.n_ckpt * (size_t)a.n_traj + (size_t)st.traj] = dt_use;
+      double* rec = ckpt_record(a.ckpt, a.ckpt_capacity, st.n_ckpt / MDX_CKPT_SEG, st.traj);
+      if (L.lane == 0) rec[MDX_NV + 1 + st.n_ckpt % MDX_CKPT_SEG] = dt_use;
       if (st.n_ckpt % MDX_CKPT_SEG == 0) {
-        double* rec = ckpt_state(a.ckpt, a.ckpt_capacity, a.n_traj, st.n_ckpt / MDX_CKPT_SEG, st.traj);
         if (L.lane == 0) rec[0] = t;
         for (int j = L.lane; j < MDX_NV; j += MDX_TEAM) rec[1 + j] = s.y[j];
       }

@@ -48,12 +48,11 @@ struct GradSlice {
 constexpr int GRAD_TEAMS_PER_BLOCK = MDX_TPB / MDX_TEAM;
 
 __device__ __forceinline__ double ckpt_h(const MdxGradArgs& a, int m, int traj) {
-  return a.ckpt[(size_t)m * (size_t)a.n_traj + (size_t)traj];
+  return ckpt_record(a.ckpt, a.ckpt_capacity, m / MDX_CKPT_SEG, traj)[MDX_NV + 1 + m % MDX_CKPT_SEG];
 }
 
 __device__ __forceinline__ const double* ckpt_seg_state(const MdxGradArgs& a, int seg, int traj) {
-  return a.ckpt + (size_t)a.ckpt_capacity * (size_t)a.n_traj +
-         ((size_t)seg * (size_t)a.n_traj + (size_t)traj) * (size_t)(MDX_NV + 1);
+  return ckpt_record(a.ckpt, a.ckpt_capacity, seg, traj);
 }
 
 __device__ __forceinline__ int last_save_reached(const double* times, int hi, double t_end) {
