@@ -49,6 +49,7 @@ extern "C" {
 #define MDX_PLAN_ADJOINT 2      /* the module carries the discrete-adjoint kernel */
 #define MDX_PLAN_SAVE_HOOK 4    /* the module calls a save hook: hook_out is required */
 #define MDX_PLAN_NO_HISTORY 8   /* the module keeps only the final state: n_save_hist == 1 */
+#define MDX_PLAN_STAGED 16     /* the module has the staged kernel (mdx_solve_staged) */
 
 /* Per-trajectory status bits written to mdx_solve_desc.status. */
 #define MDX_STATUS_OK 0
@@ -205,6 +206,16 @@ int mdx_solve_persistent_noalloc(mdx_plan* plan, const mdx_solve_desc* desc, voi
 
 /* Launch the discrete-adjoint reverse pass on `stream` (MDX_PLAN_ADJOINT plans). */
 int mdx_grad(mdx_plan* plan, const mdx_grad_desc* desc, void* stream);
+
+/* A persistent solve in two stages, for long integrations of uneven and unknown length
+ * (MDX_PLAN_STAGED plans): every trajectory takes `slice` attempted steps, then the unfinished
+ * ones go on from there, those with the most left (at their pace so far) first.  Same results as
+ * mdx_solve with MDX_LAUNCH_PERSISTENT, bit for bit; desc->mode must be that, desc->hist_host and
+ * the desc's own workspace are not used.  `workspace` is device memory of
+ * mdx_staged_workspace_size bytes, 16-byte aligned, free again when the stream is past the call. */
+int mdx_staged_workspace_size(const mdx_plan* plan, int n_traj, size_t* bytes);
+int mdx_solve_staged(mdx_plan* plan, const mdx_solve_desc* desc, int slice, void* workspace, size_t workspace_bytes,
+                     void* stream);
 
 /* The visiting order of a persistent launch (mdx_solve_desc.order): a permutation
  * of 0..n-1 by descending step count, from `steps` (n ints on the device, such as a

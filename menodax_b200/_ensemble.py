@@ -139,7 +139,7 @@ class Workspace:
 
 def launch(problem, *, y0, times, params, weights, dt0, rtol, atol, max_steps, mode,
            n_save_hist=None, grid_blocks=0, order=None, ckpt=None, ckpt_count=None,
-           ckpt_capacity=0, out=None, hook_out=None, hist_host=None):
+           ckpt_capacity=0, out=None, hook_out=None, hist_host=None, slice_steps=0):
     """Allocate outputs on ``y0``'s device and launch one ensemble solve.
 
     All inputs must already be contiguous float64 CUDA tensors on one device.
@@ -184,12 +184,18 @@ def launch(problem, *, y0, times, params, weights, dt0, rtol, atol, max_steps, m
             raise ValueError(f"hist_host must be a contiguous pinned float64 CPU tensor of shape {tuple(hist.shape)}")
         desc.hist_host = hist_host.data_ptr()
     stream = torch.cuda.current_stream(dev).cuda_stream
+    desc.grid_blocks = int(grid_blocks)
+    if slice_steps:
+        # Two stages; the scratch holds a state per trajectory, so it goes back after each call.
+        scratch = torch.empty(problem.plan.staged_workspace_size(n), dtype=torch.uint8, device=dev)
+        with torch.cuda.device(dev):
+            problem.plan.solve_staged(desc, int(slice_steps), scratch.data_ptr(), scratch.numel(), stream)
+        return hist, counters
     if mode == _native.MDX_LAUNCH_PERSISTENT:
         nbytes = problem.plan.workspace_size(mode, n)
         ws = Workspace.get(dev, stream, nbytes)
         desc.workspace = ws.data_ptr()
         desc.workspace_bytes = ws.numel()
-    desc.grid_blocks = int(grid_blocks)
     if ckpt is not None:
         desc.ckpt = ckpt.data_ptr()
         desc.ckpt_count = ckpt_count.data_ptr()

@@ -100,6 +100,7 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
     hook_out = None
     if options.save_hook is not None:
         hook_out = torch.empty((n, options.hook_size), dtype=torch.float64, device=device)
+    slice_steps = 0
     input_on_gpu = any(isinstance(x, torch.Tensor) and x.is_cuda for x in (y0, params))
     host_results = not (torch_io and input_on_gpu)
     if launch_mode == "auto" and n >= AUTOTUNE_MIN_TRAJECTORIES and hook_out is None:
@@ -111,6 +112,7 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
         problem = get_problem(ode_fn, n_vars, n_params, options)
         mode = choice.mode
         grid_blocks = autotune.grid_blocks(problem, choice, n)
+        slice_steps = autotune.slice_steps(choice)
         if host_results and autotune.streams_to_host(choice):
             mode = _native.MDX_LAUNCH_PLAIN
             grid_blocks = 0
@@ -141,14 +143,14 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
         streamed = mode == _native.MDX_LAUNCH_PLAIN
     order = None
     order_key = None
-    if mode == _native.MDX_LAUNCH_PERSISTENT:
+    if mode == _native.MDX_LAUNCH_PERSISTENT and not slice_steps:
         order_key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol),
                      int(max_steps), int(grid_blocks), stream_key(device))
         order = _order_hint.get(order_key)
         if order is not None and (order.device != device or order.numel() != n):
             order = None
     hist, counters = launch(problem, mode=mode, grid_blocks=grid_blocks, hook_out=hook_out,
-                            hist_host=hist_h if streamed else None, order=order, **common)
+                            hist_host=hist_h if streamed else None, order=order, slice_steps=slice_steps, **common)
     if order_key is not None and n > 0:
         _remember_order(order_key, longest_first(counters[2]))
     if hist_h is None:

@@ -34,6 +34,7 @@ MDX_PLAN_CHECKPOINT = 1
 MDX_PLAN_ADJOINT = 2
 MDX_PLAN_SAVE_HOOK = 4
 MDX_PLAN_NO_HISTORY = 8
+MDX_PLAN_STAGED = 16
 MDX_MAX_SHARED_BYTES = 227 * 1024
 MDX_STATUS_MAX_STEPS = 1
 MDX_STATUS_NONFINITE = 2
@@ -44,7 +45,7 @@ EXPORTED = (
     "mdx_occupancy", "mdx_solve", "mdx_grad", "mdx_last_error", "mdx_version",
     "mdx_measure_fma_peak", "mdx_solve_persistent_noalloc", "mdx_checkpoint_size",
     "mdx_order_workspace_size", "mdx_order_longest_first",
-    "mdx_sens_contract",
+    "mdx_sens_contract", "mdx_staged_workspace_size", "mdx_solve_staged",
 )
 
 
@@ -154,6 +155,9 @@ def lib():
         L.mdx_order_longest_first.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,
                                               ctypes.c_size_t, ctypes.c_void_p]
         L.mdx_sens_contract.argtypes = ([ctypes.c_void_p] * 2 + [ctypes.c_int] * 5 + [ctypes.c_void_p] * 3)
+        L.mdx_staged_workspace_size.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_size_t)]
+        L.mdx_solve_staged.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveDesc), ctypes.c_int, ctypes.c_void_p,
+                                       ctypes.c_size_t, ctypes.c_void_p]
         L.mdx_measure_fma_peak.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
         _lib = L
         return _lib
@@ -304,6 +308,16 @@ class Plan:
     def solve(self, desc: SolveDesc, stream: int):
         desc.struct_size = ctypes.sizeof(SolveDesc)
         check(lib().mdx_solve(self.handle, ctypes.byref(desc), ctypes.c_void_p(stream)), "mdx_solve")
+
+    def staged_workspace_size(self, n_traj: int) -> int:
+        out = ctypes.c_size_t()
+        check(lib().mdx_staged_workspace_size(self.handle, n_traj, ctypes.byref(out)), "mdx_staged_workspace_size")
+        return out.value
+
+    def solve_staged(self, desc: SolveDesc, slice_steps: int, workspace: int, nbytes: int, stream: int):
+        desc.struct_size = ctypes.sizeof(SolveDesc)
+        check(lib().mdx_solve_staged(self.handle, ctypes.byref(desc), slice_steps, workspace, nbytes,
+                                     ctypes.c_void_p(stream)), "mdx_solve_staged")
 
     def grad(self, desc: GradDesc, stream: int):
         desc.struct_size = ctypes.sizeof(GradDesc)

@@ -74,6 +74,9 @@ class KernelOptions:
     # With a team and a dense FP32 LU in fast arithmetic: M inverted in the lanes'
     # registers (kernels/mdx_team_inverse.cuh) instead of factorised in shared memory.
     inverse: bool = False
+    # A persistent launch in two stages (kernels/mdx_entry.cuh, mdx_solve_staged): thread and
+    # cyclic kernels of plain solves.
+    staged: bool = False
     # Tsit5: the stage vectors k1..k6 in shared memory, one column per thread
     # (the reference's "shared" backend, modax/tsit5.py:117-139).
     shared_stages: bool = False
@@ -304,6 +307,14 @@ def _build_team_source(tr, n_vars: int, n_params: int, options: KernelOptions, s
     return "\n".join(parts) + "\n", meta
 
 
+def staged_defines(options: KernelOptions) -> list[str]:
+    if not options.staged:
+        return []
+    if options.save_hook is not None or options.checkpoint or (options.team and not options.cyclic):
+        raise ValueError("staged launches are for plain solves on threads or cyclic lanes")
+    return ["#define MDX_STAGED 1", f"#define MDX_STAGE mdx::{'tsit5' if options.solver == 'tsit5' else 'rodas5p'}"]
+
+
 def _cyclic_options(options: KernelOptions) -> bool:
     """The builds the cyclic kernel covers: plain solves in fast arithmetic with a 32-bit
     sparse LU.  Its elimination is unpivoted, as the sparse LU's is, in an order of its own, so a
@@ -369,6 +380,7 @@ def _build_cyclic_source(ode_fn, tr, n_vars: int, n_params: int, options: Kernel
         f"#define MDX_SEPARATORS {len(layout.separators)}",
         f"#define MDX_LANE_PARAMS {len(layout.params)}",
         f"#define MDX_AUTONOMOUS {1 if autonomous else 0}",
+        *staged_defines(options),
         '#include "mdx_common.cuh"',
         "namespace mdx { namespace cyclic {",
         "typedef MDX_LU_T lu_t;",
@@ -432,6 +444,7 @@ def build_source(ode_fn, n_vars: int, n_params: int, options: KernelOptions):
     if options.cyclic:
         return _build_cyclic_source(ode_fn, tr, n_vars, n_params, options)
     if options.team:
+        staged_defines(options)  # refuses: the team kernel has no staged launch
         return _build_team_source(tr, n_vars, n_params, options, stage_tr)
     sens = _sens_layout(n_vars, n_params, options.sens)
     n_sens = 0 if sens is None else sens.n_sens
@@ -470,6 +483,7 @@ def build_source(ode_fn, n_vars: int, n_params: int, options: KernelOptions):
         f"#define MDX_MIN_BLOCKS {int(options.min_blocks)}",
         f"#define MDX_SOLVE_T {'double' if wide else lu_t}",
         f"#define MDX_WIDE_SOLVE {1 if wide else 0}",
+        *staged_defines(options),
         '#include "mdx_common.cuh"',
     ]
     sens_weight = "1.0" if error_control else "0.0"
@@ -608,7 +622,7 @@ def get_problem(ode_fn, n_vars: int, n_params: int, options: KernelOptions) -> P
         _native.MDX_PLAN_ADJOINT if options.adjoint else 0
     ) | (_native.MDX_PLAN_SAVE_HOOK if options.save_hook is not None else 0) | (
         0 if options.save_history else _native.MDX_PLAN_NO_HISTORY
-    )
+    ) | (_native.MDX_PLAN_STAGED if options.staged else 0)
     solver = _native.MDX_SOLVER_TSIT5 if options.solver == "tsit5" else _native.MDX_SOLVER_RODAS5P
     plan = _native.Plan(solver, n_vars, meta["n_system"], n_params, options.threads_per_block, flags, cubin,
                         ckpt_stride=int(options.ckpt_stride), team_size=max(1, int(options.team)),

@@ -42,6 +42,14 @@ typedef struct MdxSolveArgs {
   double atol;
 } MdxSolveArgs;
 
+/* A staged solve's second parameter block: every trajectory for its first steps,
+ * then the unfinished ones from where they stopped, longest first. */
+typedef struct MdxStageArgs {
+  double* records;   /* (N, record size) states between the stages */
+  int* remaining;    /* (N,) written by the first stage: steps still to take, about; 0 when finished */
+  int slice;         /* first stage: attempted steps after which a trajectory stops; 0: the second stage */
+} MdxStageArgs;
+
 typedef struct MdxGradArgs {
   const double* times;
   const double* params;

@@ -152,6 +152,45 @@ __device__ __forceinline__ bool save_reached(double ts, double t_new) {
   return ts <= t_new + 1e-12 * pymax(1.0, fabs(ts));
 }
 
+#ifndef MDX_STAGED
+#define MDX_STAGED 0
+#endif
+
+// What a trajectory that stopped after `steps` attempted steps at t still has to take,
+// if it goes on at its average pace: what the second stage is ordered by.
+__device__ __forceinline__ int steps_to_go(double t0, double t, double tf, int steps) {
+  const double more = (tf - t) / (t - t0) * (double)steps;
+  return more >= 1.0 ? (more < 1e9 ? (int)more : 1000000000) : 1;
+}
+
+// The scalars of a stopped trajectory's state, six doubles of its record.
+constexpr int RECORD_SCALARS = 6;
+template <class S>
+__device__ __forceinline__ void save_scalars(const S& st, double* rec) {
+  rec[0] = st.t;
+  rec[1] = st.dt;
+  rec[2] = st.err_prev;
+  rec[3] = st.err_prev2;
+  int* counts = reinterpret_cast<int*>(rec + 4);
+  counts[0] = st.save_idx;
+  counts[1] = st.n_steps;
+  counts[2] = st.accepted;
+  counts[3] = st.rejected;
+}
+template <class S>
+__device__ __forceinline__ void load_scalars(S& st, const MdxSolveArgs& a, const double* rec) {
+  st.t = rec[0];
+  st.dt = rec[1];
+  st.err_prev = rec[2];
+  st.err_prev2 = rec[3];
+  const int* counts = reinterpret_cast<const int*>(rec + 4);
+  st.save_idx = counts[0];
+  st.n_steps = counts[1];
+  st.accepted = counts[2];
+  st.rejected = counts[3];
+  if (st.save_idx < a.n_save) st.next_save = a.times[st.save_idx];
+}
+
 #ifndef MDX_CKPT_SEG
 #define MDX_CKPT_SEG 1
 #endif

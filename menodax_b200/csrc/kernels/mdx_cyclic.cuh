@@ -54,6 +54,7 @@ struct State {
   double y[B];
   double p[MDX_LANE_PARAMS > 0 ? MDX_LANE_PARAMS : 1];
   double t, dt, err_prev, err_prev2, tf_local;
+  double next_save;  // times[save_idx]: read when the cursor moves, not on every step
   int save_idx, n_steps, accepted, rejected, traj;
 };
 
@@ -247,7 +248,7 @@ __device__ __forceinline__ void rest(State& st) {
   for (int j = 0; j < B; ++j) st.y[j] = 0.0;
 #pragma unroll
   for (int k = 0; k < MDX_LANE_PARAMS; ++k) st.p[k] = 0.0;
-  st.t = st.tf_local = 0.0;
+  st.t = st.tf_local = st.next_save = 0.0;
   st.dt = st.err_prev = st.err_prev2 = 1.0;
   st.save_idx = st.n_steps = st.accepted = st.rejected = st.traj = 0;
 }
@@ -268,6 +269,7 @@ __device__ __forceinline__ void init(State& st, const MdxSolveArgs& a, int traj,
   st.t = t0;
   st.dt = a.dt0 > 0.0 ? a.dt0 : (tf - t0) * 1e-6;
   st.save_idx = 1;
+  st.next_save = a.times[a.n_save > 1 ? 1 : 0];
   st.n_steps = 0;
   st.accepted = 0;
   st.rejected = 0;
@@ -393,9 +395,9 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a, const Lan
     st.err_prev2 = st.err_prev;
     st.err_prev = safe_err;
     const double t_new = t + dt_use;
-    while (st.save_idx < a.n_save && save_reached(a.times[st.save_idx], t_new)) {
+    while (st.save_idx < a.n_save && save_reached(st.next_save, t_new)) {
       // The thread kernel's dense output: eight weights shared by every component.
-      const double theta = (a.times[st.save_idx] - t) * inv_dt;
+      const double theta = (st.next_save - t) * inv_dt;
       const double theta1 = 1.0 - theta;
       double w[8];
 #pragma unroll
@@ -410,6 +412,7 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a, const Lan
         row[j] = theta1 * st.y[j] + theta * (y_new + theta1 * hsum);
       }
       ++st.save_idx;
+      if (st.save_idx < a.n_save) st.next_save = a.times[st.save_idx];
     }
 #pragma unroll
     for (int j = 0; j < B; ++j) st.y[j] = u[j] + (double)k[7][j];
@@ -453,6 +456,71 @@ __device__ __forceinline__ void finish(State& st, const MdxSolveArgs& a, const L
     for (size_t i = L.lane; i < row; i += MDX_TEAM) dst[i] = __ldcg(src + i);
   }
 }
+
+#if MDX_STAGED
+// A stopped trajectory's record: its scalars, then the state; every lane has the scalars.
+constexpr int RECORD = RECORD_SCALARS + MDX_NV;
+__device__ __forceinline__ void save(const State& st, double* rec, const Lane& L) {
+  if (L.lane == 0) save_scalars(st, rec);
+#pragma unroll
+  for (int j = 0; j < B; ++j) rec[RECORD_SCALARS + L.lane * B + j] = st.y[j];
+}
+__device__ __forceinline__ void load(State& st, const MdxSolveArgs& a, const double* rec, int traj, const Lane& L) {
+  st.traj = traj;
+#pragma unroll
+  for (int j = 0; j < B; ++j) st.y[j] = rec[RECORD_SCALARS + L.lane * B + j];
+#pragma unroll
+  for (int k = 0; k < MDX_LANE_PARAMS; ++k) st.p[k] = a.params[(size_t)traj * MDX_NP + param_column(k, L.lane)];
+#if MDX_TF_INDEX >= 0
+  st.tf_local = a.params[(size_t)traj * MDX_NP + MDX_TF_INDEX];
+#else
+  st.tf_local = a.times[a.n_save - 1];
+#endif
+  load_scalars(st, a, rec);
+}
+
+// The two stages of mdx_entry.cuh's mdx_solve_staged, a trajectory per team.
+__device__ __forceinline__ void solve_staged(const MdxSolveArgs& a, const MdxStageArgs& b) {
+  const Lane L = lane_of_thread();
+  State st;
+  rest(st);
+  bool active = false, drained = false;
+  while (true) {
+    const bool whole = active && !running(st, a);
+    if (__any_sync(MDX_FULL_MASK, whole)) finish(st, a, L, whole);
+    if (b.slice > 0 && active && (whole || st.n_steps >= b.slice)) {
+      if (L.lane == 0) b.remaining[st.traj] = whole ? 0 : steps_to_go(a.times[0], st.t, st.tf_local, st.n_steps);
+      if (!whole) save(st, b.records + (size_t)st.traj * RECORD, L);
+      active = false;
+    }
+    active = active && !whole;
+    if (__any_sync(MDX_FULL_MASK, !active && !drained)) {
+      int slot = 0;
+      if (!active && !drained && L.lane == 0) slot = atomicAdd(a.work_counter, 1);
+      slot = __shfl_sync(MDX_FULL_MASK, slot, L.base);
+      if (!active && !drained) {
+        if (slot >= a.n_traj) {
+          drained = true;
+        } else {
+          const int traj = a.order ? a.order[slot] : slot;
+          if (b.slice > 0) {
+            init(st, a, traj, L);
+            active = true;
+          } else if (b.remaining[traj] > 0) {
+            load(st, a, b.records + (size_t)traj * RECORD, traj, L);
+            active = true;
+          } else {
+            drained = true;  // finished ones come last in the order
+          }
+        }
+      }
+      continue;
+    }
+    if (!__any_sync(MDX_FULL_MASK, active)) break;
+    step(st, a, L, active);
+  }
+}
+#endif
 
 // REFILL: lanes whose trajectory ends take the next one off the queue (one
 // atomicAdd per trajectory, by its first lane); nothing waits on anything.
@@ -503,3 +571,10 @@ extern "C" __global__ void __launch_bounds__(MDX_TPB, MDX_MIN_BLOCKS) mdx_solve_
 extern "C" __global__ void __launch_bounds__(MDX_TPB, MDX_MIN_BLOCKS) mdx_solve_persistent(const MdxSolveArgs a) {
   mdx::cyclic::solve_warp<true>(a);
 }
+
+#if MDX_STAGED
+extern "C" __global__ void __launch_bounds__(MDX_TPB, MDX_MIN_BLOCKS)
+mdx_solve_staged(const MdxSolveArgs a, const MdxStageArgs b) {
+  mdx::cyclic::solve_staged(a, b);
+}
+#endif

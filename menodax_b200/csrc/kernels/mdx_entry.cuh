@@ -103,3 +103,57 @@ mdx_solve_persistent(const MdxSolveArgs a) {
     if (active && MDX_SOLVER::running(st, a)) MDX_SOLVER::step(st, a);
   }
 }
+
+#if MDX_STAGED
+// The persistent launch in two stages (MdxStageArgs).  The first takes every trajectory
+// `slice` steps from its start and leaves the unfinished ones in `records`; the
+// second, given the order of what remains, takes them on from there, longest first.
+// Where step counts are uneven and not known beforehand, a long integration that
+// happened to start late would run on alone after the rest; an integration does not
+// depend on when it runs, so the results are the persistent launch's bit for bit.
+extern "C" __global__ void __launch_bounds__(MDX_TPB, MDX_MIN_BLOCKS)
+mdx_solve_staged(const MdxSolveArgs a, const MdxStageArgs b) {
+  const unsigned lane = threadIdx.x & 31u;
+  const unsigned lanes_below = (1u << lane) - 1u;
+  MDX_SOLVER::State st;
+  bool active = false;
+  bool drained = false;
+  while (true) {
+    const bool whole = active && !MDX_SOLVER::running(st, a);
+    if (whole) MDX_SOLVER::finish(st, a);
+    if (b.slice > 0 && active && (whole || st.n_steps >= b.slice)) {
+      b.remaining[st.traj] = whole ? 0 : mdx::steps_to_go(a.times[0], st.t, MDX_STAGE::end_time(st), st.n_steps);
+      if (!whole) MDX_STAGE::save(st, b.records + (size_t)st.traj * MDX_STAGE::RECORD);
+      active = false;
+    }
+    if (whole) active = false;
+    const unsigned idle = __ballot_sync(MDX_FULL_MASK, !active);
+    if (idle != 0u && !drained) {
+      const int leader = __ffs(idle) - 1;
+      const int want = __popc(idle);
+      int base = 0;
+      if ((int)lane == leader) base = atomicAdd(a.work_counter, want);
+      base = __shfl_sync(MDX_FULL_MASK, base, leader);
+      if (!active) {
+        const int slot = base + __popc(idle & lanes_below);
+        if (slot < a.n_traj) {
+          const int traj = a.order ? a.order[slot] : slot;
+          if (b.slice > 0) {
+            MDX_SOLVER::init(st, a, traj);
+            active = true;
+          } else if (b.remaining[traj] > 0) {  // finished ones come last in the order
+            MDX_STAGE::load(st, a, b.records + (size_t)traj * MDX_STAGE::RECORD, traj);
+            active = true;
+          }
+        }
+      }
+      if (base + want >= a.n_traj) drained = true;
+    }
+    if (!__any_sync(MDX_FULL_MASK, active)) {
+      if (drained) break;
+      continue;
+    }
+    if (active && MDX_SOLVER::running(st, a)) MDX_SOLVER::step(st, a);
+  }
+}
+#endif

@@ -438,6 +438,29 @@ __device__ __forceinline__ void finish(State& st, const MdxSolveArgs& a) {
   }
 }
 
+#if MDX_STAGED
+constexpr int RECORD = RECORD_SCALARS + MDX_NS;
+__device__ __forceinline__ void save(const State& st, double* rec) {
+  save_scalars(st, rec);
+#pragma unroll
+  for (int j = 0; j < MDX_NS; ++j) rec[RECORD_SCALARS + j] = st.y[j];
+}
+__device__ __forceinline__ void load(State& st, const MdxSolveArgs& a, const double* rec, int traj) {
+  st.traj = traj;
+#pragma unroll
+  for (int j = 0; j < MDX_NS; ++j) st.y[j] = rec[RECORD_SCALARS + j];
+#pragma unroll
+  for (int k = 0; k < MDX_NP; ++k) st.p[k] = a.params[(size_t)traj * MDX_NP + k];
+#if MDX_TF_INDEX >= 0
+  st.tf_local = st.p[MDX_TF_INDEX];
+#else
+  st.tf_local = a.times[a.n_save - 1];
+#endif
+  load_scalars(st, a, rec);
+}
+__device__ __forceinline__ double end_time(const State& st) { return st.tf_local; }
+#endif
+
 }  // namespace rodas5p
 
 struct Rodas5P {

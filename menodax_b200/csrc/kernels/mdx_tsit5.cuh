@@ -271,6 +271,31 @@ __device__ __forceinline__ void finish(State& st, const MdxSolveArgs& a) {
   }
 }
 
+#if MDX_STAGED
+constexpr int RECORD = RECORD_SCALARS + 2 * MDX_NS;
+__device__ __forceinline__ void save(const State& st, double* rec) {
+  save_scalars(st, rec);
+#pragma unroll
+  for (int j = 0; j < MDX_NS; ++j) {
+    rec[RECORD_SCALARS + j] = st.y[j];
+    rec[RECORD_SCALARS + MDX_NS + j] = st.k7[j];
+  }
+}
+__device__ __forceinline__ void load(State& st, const MdxSolveArgs& a, const double* rec, int traj) {
+  st.traj = traj;
+#pragma unroll
+  for (int j = 0; j < MDX_NS; ++j) {
+    st.y[j] = rec[RECORD_SCALARS + j];
+    st.k7[j] = rec[RECORD_SCALARS + MDX_NS + j];
+  }
+#pragma unroll
+  for (int k = 0; k < MDX_NP; ++k) st.p[k] = a.params[(size_t)traj * MDX_NP + k];
+  st.tf = a.times[a.n_save - 1];
+  load_scalars(st, a, rec);
+}
+__device__ __forceinline__ double end_time(const State& st) { return st.tf; }
+#endif
+
 }  // namespace tsit5
 
 struct Tsit5 {

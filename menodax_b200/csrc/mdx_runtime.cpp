@@ -161,6 +161,7 @@ struct Loaded {
   CUmodule module = nullptr;
   CUfunction plain = nullptr;
   CUfunction persistent = nullptr;
+  CUfunction staged = nullptr;   // MDX_PLAN_STAGED modules
   CUfunction grad = nullptr;
   CUfunction combine = nullptr;  // thread adjoint modules: the split reverse's composition
   int sm_count = 0;
@@ -211,6 +212,9 @@ int load_for_context(mdx_plan* plan, Loaded** out) {
     return cuda_fail(r, "cuModuleGetFunction(mdx_solve_plain)");
   if ((r = g_driver.moduleGetFunction(&l.persistent, guard.module, "mdx_solve_persistent")) != CUDA_SUCCESS)
     return cuda_fail(r, "cuModuleGetFunction(mdx_solve_persistent)");
+  if ((plan->desc.flags & MDX_PLAN_STAGED) &&
+      (r = g_driver.moduleGetFunction(&l.staged, guard.module, "mdx_solve_staged")) != CUDA_SUCCESS)
+    return cuda_fail(r, "cuModuleGetFunction(mdx_solve_staged)");
   if (plan->desc.flags & MDX_PLAN_ADJOINT) {
     if ((r = g_driver.moduleGetFunction(&l.grad, guard.module, "mdx_grad_reverse")) != CUDA_SUCCESS)
       return cuda_fail(r, "cuModuleGetFunction(mdx_grad_reverse)");
@@ -440,7 +444,7 @@ namespace mdx_internal {
 
 // The body of mdx_solve.  `counter` (when not NULL) replaces the caller's
 // workspace as the persistent kernel's queue head.
-int solve_with_counter(mdx_plan* plan, const mdx_solve_desc* d, void* stream, int* counter) {
+int solve_with_counter(mdx_plan* plan, const mdx_solve_desc* d, void* stream, int* counter, const Stage* stage) {
   if (!plan || !d) return fail(MDX_E_INVALID, "mdx_solve: null argument");
   if (d->struct_size != (int)sizeof(mdx_solve_desc))
     return fail(MDX_E_INVALID, "mdx_solve_desc.struct_size %d != %d", d->struct_size, (int)sizeof(mdx_solve_desc));
@@ -526,6 +530,24 @@ int solve_with_counter(mdx_plan* plan, const mdx_solve_desc* d, void* stream, in
     CUresult r = g_driver.memsetD32Async((CUdeviceptr)a.work_counter, 0u, 1, s);
     if (r != CUDA_SUCCESS) return cuda_fail(r, "cuMemsetD32Async(work counter)");
   }
+  if (stage) {
+    MdxStageArgs b;
+    b.records = stage->records;
+    b.remaining = stage->remaining;
+    b.slice = stage->slice;
+    void* staged[] = {&a, &b};
+    CUresult r = g_driver.launchKernel(l->staged, grid, 1, 1, tpb, 1, 1, smem, s, staged, nullptr);
+    if (r != CUDA_SUCCESS) return cuda_fail(r, "cuLaunchKernel(mdx_solve_staged)");
+    if ((rc = mdx_order_longest_first(stage->remaining, d->n_traj, stage->order, stage->sort, stage->sort_bytes, stream)))
+      return rc;
+    if ((r = g_driver.memsetD32Async((CUdeviceptr)a.work_counter, 0u, 1, s)) != CUDA_SUCCESS)
+      return cuda_fail(r, "cuMemsetD32Async(work counter)");
+    a.order = stage->order;
+    b.slice = 0;
+    r = g_driver.launchKernel(l->staged, grid, 1, 1, tpb, 1, 1, smem, s, staged, nullptr);
+    if (r != CUDA_SUCCESS) return cuda_fail(r, "cuLaunchKernel(mdx_solve_staged)");
+    return MDX_OK;
+  }
   void* params[] = {&a};
   CUresult r = g_driver.launchKernel(f, grid, 1, 1, tpb, 1, 1, smem, s, params, nullptr);
   if (r != CUDA_SUCCESS) return cuda_fail(r, "cuLaunchKernel(mdx_solve)");
@@ -557,6 +579,65 @@ extern "C" {
 
 int mdx_solve(mdx_plan* plan, const mdx_solve_desc* d, void* stream) {
   return mdx_internal::solve_with_counter(plan, d, stream, nullptr);
+}
+
+}  // extern "C"
+
+namespace {
+
+// Where a staged solve's scratch lies in its workspace: the queue head, the sort's
+// scratch, the steps remaining, the order, the records.
+struct StageLayout {
+  size_t sort_bytes, sort, remaining, order, records, total;
+};
+
+StageLayout stage_layout(const mdx_plan* plan, int n_traj) {
+  // A record is six doubles of scalars and the state, for Tsit5 its first stage too
+  // (RECORD in the kernels).
+  const size_t state = (size_t)plan->desc.n_system * (plan->desc.solver == MDX_SOLVER_TSIT5 ? 2 : 1);
+  auto aligned = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  StageLayout l;
+  mdx_order_workspace_size(&l.sort_bytes);
+  l.sort = 256;
+  l.remaining = aligned(l.sort + l.sort_bytes);
+  l.order = aligned(l.remaining + sizeof(int) * (size_t)n_traj);
+  l.records = aligned(l.order + sizeof(int) * (size_t)n_traj);
+  l.total = l.records + sizeof(double) * (6 + state) * (size_t)n_traj;
+  return l;
+}
+
+}  // namespace
+
+extern "C" {
+
+int mdx_staged_workspace_size(const mdx_plan* plan, int n_traj, size_t* bytes) {
+  if (!plan || !bytes) return fail(MDX_E_INVALID, "mdx_staged_workspace_size: null argument");
+  if (n_traj < 0) return fail(MDX_E_INVALID, "n_traj must be non-negative");
+  *bytes = stage_layout(plan, n_traj).total;
+  return MDX_OK;
+}
+
+int mdx_solve_staged(mdx_plan* plan, const mdx_solve_desc* d, int slice, void* workspace, size_t workspace_bytes,
+                     void* stream) {
+  if (!plan || !d) return fail(MDX_E_INVALID, "mdx_solve_staged: null argument");
+  if (!(plan->desc.flags & MDX_PLAN_STAGED)) return fail(MDX_E_INVALID, "the plan was built without the staged kernel");
+  if (d->struct_size != (int)sizeof(mdx_solve_desc))
+    return fail(MDX_E_INVALID, "mdx_solve_desc.struct_size %d != %d", d->struct_size, (int)sizeof(mdx_solve_desc));
+  if (d->mode != MDX_LAUNCH_PERSISTENT || d->hist_host)
+    return fail(MDX_E_INVALID, "a staged solve is a persistent one without a host history");
+  if (slice < 1 || d->n_traj < 0) return fail(MDX_E_INVALID, "mdx_solve_staged: slice %d, n_traj %d", slice, d->n_traj);
+  const StageLayout l = stage_layout(plan, d->n_traj);
+  if (d->n_traj > 0 && (!workspace || workspace_bytes < l.total || ((size_t)workspace & 15)))
+    return fail(MDX_E_INVALID, "mdx_solve_staged needs %zu bytes of 16-byte aligned workspace", l.total);
+  char* w = (char*)workspace;
+  mdx_internal::Stage stage;
+  stage.slice = slice;
+  stage.sort = w + l.sort;
+  stage.sort_bytes = l.sort_bytes;
+  stage.remaining = (int*)(w + l.remaining);
+  stage.order = (int*)(w + l.order);
+  stage.records = (double*)(w + l.records);
+  return mdx_internal::solve_with_counter(plan, d, stream, (int*)workspace, &stage);
 }
 
 int mdx_grad(mdx_plan* plan, const mdx_grad_desc* d, void* stream) {

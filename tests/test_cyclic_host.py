@@ -54,6 +54,11 @@ def _system(name, points, size):
     if name == "brusselator":
         cfg = systems.brusselator_config(points, size=size)
         return cfg["ode_fn"], 2 * points, 1, cfg["sparsity"], cfg["y0"], cfg["params"], np.linspace(0.0, 4.0, 7)
+    if name == "bare":  # no parameters at all
+        fn, mask = forced_chain(points)
+        bare = lambda y, t, p: fn(y, t, [3.0] + [1.0] * points)  # noqa: E731
+        return bare, points, 0, mask, np.random.default_rng(4).normal(1.0, 0.3, (size, points)), np.zeros((size, 0)), \
+            np.linspace(0.0, 1.5, 6)
     fn, mask = forced_chain(points)
     rng = np.random.default_rng(3)
     params = np.concatenate([rng.uniform(5.0, 20.0, (size, 1)), rng.uniform(0.5, 2.0, (size, points))], axis=1)
@@ -95,6 +100,7 @@ def _thread_kernel(tmp_path, fn, n_vars, n_params, mask, **kw):
     ("brusselator", 32, 32),
     ("forced", 12, 4),         # one separator; explicit time; a parameter that moves with the block
     ("forced", 16, 16),        # blocks of one component
+    ("bare", 8, 4),
 ])
 def test_cyclic_steps_like_the_thread_kernel(tmp_path, name, points, lanes):
     fn, n_vars, n_params, mask, y0, params, times = _system(name, points, size=9)   # a partly filled last warp

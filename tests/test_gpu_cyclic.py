@@ -61,3 +61,16 @@ def test_every_lane_count_and_launch(name):
         for kw in (dict(grid_blocks=3), dict(order=order)):
             again, c = launch(problem, mode=_native.MDX_LAUNCH_PERSISTENT, **kw, **common)
             assert torch.equal(again, hist) and torch.equal(c, counters)
+
+
+def test_error_weights_and_own_end_times():
+    """Weights and end times per trajectory: the FP64 thread kernel's answer within 20 rtol."""
+    cfg, n = _config("brusselator", 300)
+    rng = np.random.default_rng(2)
+    params = np.concatenate([cfg["params"], rng.uniform(1.0, 3.0, (300, 1))], axis=1)
+    args = (cfg["ode_fn"], cfg["y0"], cfg["t_span"], params)
+    kw = dict(rtol=cfg["rtol"], atol=cfg["atol"], sparsity=cfg["sparsity"], tf_index=1,
+              error_weights=rng.uniform(0.5, 1.5, (300, n)))
+    hist = rodas5P.solve(*args, **kw)
+    ref = rodas5P.solve(*args, lu_precision="fp64", team=0, launch="plain", **kw)
+    assert (np.abs(hist - ref) / np.abs(ref).max(axis=(1, 2), keepdims=True)).max() <= 20 * cfg["rtol"]
