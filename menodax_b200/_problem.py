@@ -315,11 +315,14 @@ def staged_defines(options: KernelOptions) -> list[str]:
     return ["#define MDX_STAGED 1", f"#define MDX_STAGE mdx::{'tsit5' if options.solver == 'tsit5' else 'rodas5p'}"]
 
 
-def _cyclic_options(options: KernelOptions) -> bool:
+def _cyclic_options(options: KernelOptions, n_vars: int) -> bool:
     """The builds the cyclic kernel covers: plain solves in fast arithmetic with a 32-bit
-    sparse LU.  Its elimination is unpivoted, as the sparse LU's is, in an order of its own, so a
+    sparse LU, of more states than the thread kernel solves in double by default (its 32-bit
+    solves move an 8-state ring's answers over [0, 300] by 4e-3 of their norm, more than a
+    last bit does).  Its elimination is unpivoted, as the sparse LU's is, in an order of its own, so a
     dense solve (which pivots) and the reference's arithmetic keep their kernels."""
     return (options.solver == "rodas5P" and options.fast and options.lu_precision == "fp32"
+            and n_vars > WIDE_SOLVE_MAX_VARS and not options.wide_solve
             and options.sparsity is not None and options.sparse_code == "auto" and options.ordering == "amd"
             and options.sens is None and options.save_hook is None and options.array_rhs is None
             and not options.checkpoint and not options.adjoint and options.save_history)
@@ -343,7 +346,7 @@ def cyclic_lanes(ode_fn, n_vars: int, n_params: int, options: KernelOptions) -> 
     """The lane counts the cyclic kernel can give a trajectory of this system: those
     that cut it into equal blocks with the same right-hand side (``_cyclic.analyse``), whose
     Jacobian the pattern covers.  Empty for any other system or build."""
-    if not _cyclic_options(options):
+    if not _cyclic_options(options, n_vars):
         return ()
     return tuple(sorted(_cyclic_layouts(ode_fn, n_vars, n_params, options.sparsity)))
 

@@ -93,14 +93,14 @@ def _thread_kernel(tmp_path, fn, n_vars, n_params, mask, **kw):
 
 
 @pytest.mark.parametrize("name,points,lanes", [
-    ("ring", 4, 4),            # separators only
+    ("ring", 8, 8),            # separators only
     ("ring", 12, 4),           # blocks of 6, odd interior chains
     ("ring", 16, 8),
     ("brusselator", 12, 4),
     ("brusselator", 32, 32),
     ("forced", 12, 4),         # one separator; explicit time; a parameter that moves with the block
     ("forced", 16, 16),        # blocks of one component
-    ("bare", 8, 4),
+    ("bare", 12, 4),
 ])
 def test_cyclic_steps_like_the_thread_kernel(tmp_path, name, points, lanes):
     fn, n_vars, n_params, mask, y0, params, times = _system(name, points, size=9)   # a partly filled last warp
@@ -190,5 +190,7 @@ def test_only_repeating_systems_have_it():
     wide, _ = systems.make_vdp_system(16, coupling_range=5)                       # reaches past the next block
     assert 8 not in lanes(wide, np.ones((32, 32), bool), 32)
     odd = lambda y, t, p: tuple(  # noqa: E731
-        p[0] * (y[(i + 1) % 8] - y[i]) * (2.0 if i == 3 else 1.0) for i in range(8))
-    assert lanes(odd, np.ones((8, 8), bool), 8) == ()
+        p[0] * (y[(i + 1) % 16] - y[i]) * (2.0 if i == 3 else 1.0) for i in range(16))
+    assert lanes(odd, np.ones((16, 16), bool), 16) == ()
+    small = systems.vdp_ring_config(4, size=1)                                    # solved in double on threads
+    assert lanes(small["ode_fn"], small["sparsity"], 8) == ()
