@@ -107,7 +107,8 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
         from menodax_b200 import autotune
 
         choice = autotune.tune(ode_fn, n_vars, n_params, options, tune_block=tune_block,
-                               tune_team=tune_team, tune_shared=tune_shared, tune_registers=tune_team, **common)
+                               tune_team=tune_team, tune_shared=tune_shared, tune_registers=tune_team,
+                               tune_orders=True, **common)
         options = autotune.options_for(options, choice)
         problem = get_problem(ode_fn, n_vars, n_params, options)
         mode = choice.mode

@@ -158,9 +158,9 @@ def grid_blocks(problem, choice: LaunchChoice, n: int) -> int:
 # Attempted steps of a staged launch's first stage: enough past an integration's start for
 # its pace to tell, a small part of the long integrations it is for.
 STAGE_STEPS = 128
-# Rings of 8 states on a B200, in index order / staged: t in [0, 300] 30.9 / 28.4 ms, [0,
-# 3000] 267 / 238 (ordered by exact step counts 244); 32 states, whose longest
-# trajectories set the time in any order, 22.9 / 23.2.
+# Rings on a B200, in index order / staged: 8 states on threads, t in [0, 300] 35.1 /
+# 29.6 ms, [0, 3000] 287 / 253 (ordered by exact step counts 249); 32 states on cyclic
+# lanes, whose longest trajectories set the time in any order, 22.9 / 23.2.
 STAGE_GAIN = 0.03
 
 
@@ -213,6 +213,16 @@ def _timed_launch(problem, choice, stream, *, n, y0, times, params, weights, dt0
     e1.record(stream)
     e1.synchronize()
     return e0.elapsed_time(e1) * 1e-3, counters
+
+
+def _timed_sort(steps, stream) -> float:
+    longest_first(steps)
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record(stream)
+    longest_first(steps)
+    e1.record(stream)
+    e1.synchronize()
+    return e0.elapsed_time(e1) * 1e-3
 
 
 def _fastest_in_full(problem_for, stream, n, max_steps, inputs, choice, buildable):
@@ -281,7 +291,7 @@ def _spread(lanes, n: int) -> int:
 
 def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, rtol, atol,
          max_steps, n_save_hist=None, tune_block=True, tune_team=False, tune_shared=False,
-         tune_registers=False):
+         tune_registers=False, tune_orders=False):
     """The fastest launch for this problem on these inputs (device tensors).
 
     With ``tune_block=False`` the block size stays ``options.threads_per_block``
@@ -291,6 +301,10 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
     With ``tune_registers`` so are the kernels that keep a trajectory in its lanes'
     registers, where they apply: the cyclic kernel, and for dense systems the team
     kernel's register inverse in place of its shared-memory LU.
+    With ``tune_orders`` a persistent launch counts as the front end's calls of it will
+    run: half of them on inputs like the last call's, longest first, half on inputs of which no
+    order is known, each followed by the sort for the next.  Robertson, 65,536 trajectories
+    on a B200: 331 and 372 us and 11 for the sort, against 356 for the one-launch kernel.
     With ``tune_shared`` (Tsit5) the launches with the stage vectors in shared
     memory are candidates beside the register ones; ``options.shared_stages``
     already set keeps them there.
@@ -305,7 +319,8 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
     trajectories finish."""
     n = y0.shape[0]
     # A call that was tuned before needs none of the candidates.
-    call = (ode_fn, n_vars, n_params, options, n, max_steps, y0.device, tune_block, tune_team, tune_shared, tune_registers)
+    call = (ode_fn, n_vars, n_params, options, n, max_steps, y0.device, tune_block, tune_team, tune_shared, tune_registers,
+            tune_orders)
     with _lock:
         found = _cache.get(call)
     if found is None:
@@ -317,7 +332,7 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
 
 
 def _tuned(call, *, y0, times, params, weights, dt0, rtol, atol, n_save_hist):
-    ode_fn, n_vars, n_params, options, n, max_steps, _, tune_block, tune_team, tune_shared, tune_registers = call
+    ode_fn, n_vars, n_params, options, n, max_steps, _, tune_block, tune_team, tune_shared, tune_registers, tune_orders = call
     if options.team:
         blocks, teams = (), ((options.team, options.threads_per_block),)
     else:
@@ -350,7 +365,7 @@ def _tuned(call, *, y0, times, params, weights, dt0, rtol, atol, n_save_hist):
         solves = (False, True)
     cands = candidates(blocks, teams, shared_blocks, options.shared_stages, solves, cyclic, inverse)
     key = (ode_fn, n_vars, n_params, replace(options, threads_per_block=32, team=0, shared_stages=False), n,
-           tuple(cands), max_steps, torch.cuda.get_device_name(y0.device))
+           tuple(cands), max_steps, torch.cuda.get_device_name(y0.device), tune_orders)
     with _lock:
         found = _cache.get(key)
     if found is not None:
@@ -405,13 +420,21 @@ def _tuned(call, *, y0, times, params, weights, dt0, rtol, atol, n_save_hist):
     # Persistent candidates are timed as the front end runs them once a problem
     # has been solved: longest first by the probe's step counts, so each warp
     # takes trajectories of about the same length.
-    order = longest_first(counters[2][:sample])
+    steps = counters[2][:sample].contiguous()
+    order = longest_first(steps)
+    sort_s = _timed_sort(steps, stream) if tune_orders else 0.0
     best = None
     for choice in buildable:
         prob = problem_for(choice)
         visit = order if choice.mode == _native.MDX_LAUNCH_PERSISTENT else None
-        _timed_launch(prob, choice, stream, n=sample, max_steps=max_steps, order=visit, **inputs)
-        secs, _ = _timed_launch(prob, choice, stream, n=sample, max_steps=max_steps, order=visit, **inputs)
+
+        def timed(visit):
+            return _timed_launch(prob, choice, stream, n=sample, max_steps=max_steps, order=visit, **inputs)[0]
+
+        timed(visit)
+        secs = timed(visit)
+        if tune_orders and visit is not None:
+            secs = 0.5 * (secs + timed(None)) + sort_s
         if best is None or secs < best[0]:
             best = (secs, choice)
     with _lock:
