@@ -15,6 +15,10 @@
 // few trajectories are left, instruction issue while the device is full.  The team
 // kernel (mdx_team.cuh) factorises and solves on one lane of a trajectory out of
 // shared memory; here all lanes work on every phase and nothing leaves registers.
+// Calls on a B200, that kernel / this: 32-state Van der Pol ring, 8,192 trajectories,
+// 110.9 / 22.8 ms (16 lanes); 64-state Brusselator, 16,384, 16.7 / 3.25 ms (8 lanes;
+// FP64 pipe 34%, conversions 25% of peak at the 1.9 warps a scheduler that 255
+// registers leave; 16 lanes 3.6, 32 lanes 4.8).
 //
 // The whole warp steps together: lanes whose trajectory is done step on stale
 // values and commit nothing, so every shuffle names the full warp.

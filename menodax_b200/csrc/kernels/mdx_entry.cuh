@@ -111,6 +111,9 @@ mdx_solve_persistent(const MdxSolveArgs a) {
 // Where step counts are uneven and not known beforehand, a long integration that
 // happened to start late would run on alone after the rest; an integration does not
 // depend on when it runs, so the results are the persistent launch's bit for bit.
+// 8-state Van der Pol ring on a B200, 32,768 trajectories at half fill, in index order
+// / in two stages / ordered by exact step counts: t in [0, 300] 35.1 / 29.6 / 29.0 ms,
+// [0, 3000] 287 / 253 / 249.
 extern "C" __global__ void __launch_bounds__(MDX_TPB, MDX_MIN_BLOCKS)
 mdx_solve_staged(const MdxSolveArgs a, const MdxStageArgs b) {
   const unsigned lane = threadIdx.x & 31u;
