@@ -317,9 +317,8 @@ def staged_defines(options: KernelOptions) -> list[str]:
 
 def _cyclic_options(options: KernelOptions, n_vars: int) -> bool:
     """The builds the cyclic kernel covers: plain solves in fast arithmetic with a 32-bit
-    sparse LU, of more states than the thread kernel solves in double by default (its 32-bit
-    solves move an 8-state ring's answers over [0, 300] by 4e-3 of their norm, more than a
-    last bit does).  Its elimination is unpivoted, as the sparse LU's is, in an order of its own, so a
+    sparse LU, of more states than the thread kernel solves in double by default (smaller
+    ones keep that kernel; this one solves in double too).  Its elimination is unpivoted, as the sparse LU's is, in an order of its own, so a
     dense solve (which pivots) and the reference's arithmetic keep their kernels."""
     return (options.solver == "rodas5P" and options.fast and options.lu_precision == "fp32"
             and n_vars > WIDE_SOLVE_MAX_VARS and not options.wide_solve

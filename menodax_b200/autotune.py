@@ -254,8 +254,8 @@ def small_choice(ode_fn, n_vars, n_params, options, n) -> LaunchChoice | None:
 
     Such an ensemble leaves the device idle, so a cyclic system takes the most lanes
     a trajectory that still give every scheduler of the device at most two warps (512
-    trajectories on a B200, 4 / 8 / 16 / 32 lanes: the 32-state ring 22.0 / 16.5 / 13.7
-    ms / --, the 64-state Brusselator -- / 0.79 / 0.52 / 0.42 ms; on the shared-memory teams
+    trajectories on a B200, 4 / 8 / 16 / 32 lanes: the 32-state ring 25.2 / 19.3 / 15.3
+    ms / --, the 64-state Brusselator -- / 0.90 / 0.65 / 0.51 ms; on the shared-memory teams
     64.4 and 3.5 ms, on threads slower still).  Other systems of ``TEAM_MIN_VARS`` states or
     more take a team by the same rule: a thread's vectors no longer fit its registers, nor a
     dense matrix at all (256 trajectories: dense 32 states 94.6 ms on threads, 4.2 on

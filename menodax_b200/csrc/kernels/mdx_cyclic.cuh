@@ -5,10 +5,15 @@
 // lane runs the same straight-line code on MDX_BLOCK components of its own, with
 // the state, the eight stage increments and the factors in its registers; a
 // neighbour's seam components come by shuffle.  The step is the thread kernel's
-// (mdx_rodas5p.cuh) in fast arithmetic, with its types: state, right-hand side,
-// Jacobian, stage sums, error and controller in double, matrix, factors, solver
-// right-hand side and increments in MDX_LU_T.  Only the order of elimination and
-// of the error sum differ.
+// (mdx_rodas5p.cuh) in fast arithmetic with its FP64 solves (MDX_WIDE_SOLVE): matrix and
+// factorisation in MDX_LU_T, the factors widened once per step, everything else in
+// double.  Only the order of elimination and of the error sum differ.
+//
+// Solves in MDX_LU_T are 7% to 30% faster and further from the FP64-LU solve than
+// the team and thread kernels' own in FP32, whose elimination orders differ: Van der Pol
+// rings, 512 trajectories, distance over the result's norm with FP32 / FP64 solves here and
+// in the thread kernel: 32 states over [0, 100] 2.5e-4 to 3.0e-4 / 1.1e-4 and 2.2e-4 / 1.1e-4,
+// 16 states over [0, 300] 1.2e-3 / 2.9e-4 to 3.9e-4 and 1.5e-3 / 3.7e-4.
 //
 // What bounds it: the step's dependent chain (a stage is a right-hand side, a
 // tableau row, the interior's substitutions and log2(MDX_TEAM) exchanges) while
@@ -16,9 +21,9 @@
 // kernel (mdx_team.cuh) factorises and solves on one lane of a trajectory out of
 // shared memory; here all lanes work on every phase and nothing leaves registers.
 // Calls on a B200, that kernel / this: 32-state Van der Pol ring, 8,192 trajectories,
-// 110.9 / 22.8 ms (16 lanes); 64-state Brusselator, 16,384, 16.7 / 3.25 ms (8 lanes;
-// FP64 pipe 34%, conversions 25% of peak at the 1.9 warps a scheduler that 255
-// registers leave; 16 lanes 3.6, 32 lanes 4.8).
+// 110.9 / 24.0 ms (8 lanes; FP32 solves 22.4, the factorisation in FP64 too 28.3);
+// 64-state Brusselator, 16,384, 16.7 / 4.0 ms (8 lanes, 255 registers and 0.8 KB of spills a
+// thread; 16 lanes 4.5, 32 lanes 7.3; FP32 solves 3.1, all in FP64 4.6).
 //
 // The whole warp steps together: lanes whose trajectory is done step on stale
 // values and commit nothing, so every shuffle names the full warp.
@@ -44,15 +49,6 @@ constexpr int LEVELS = MDX_TEAM == 32 ? 5 : MDX_TEAM == 16 ? 4 : MDX_TEAM == 8 ?
 static_assert(MDX_TEAM == 4 || MDX_TEAM == 8 || MDX_TEAM == 16 || MDX_TEAM == 32, "4, 8, 16 or 32 lanes");
 static_assert(MDX_TPB % 32 == 0, "blocks are whole warps");
 static_assert(B * MDX_TEAM == MDX_NV && MDX_NS == MDX_NV, "equal blocks of the plain system");
-
-// Increments are rounded to the LU type.  Blocks of up to four components keep
-// them widened (each is read by every later stage: a conversion per read costs
-// more than the registers); larger blocks would spill.
-#if MDX_BLOCK <= 4
-typedef double k_t;
-#else
-typedef lu_t k_t;
-#endif
 
 struct State {
   double y[B];
@@ -89,8 +85,7 @@ __device__ __forceinline__ void multiply(const Block& a, const Block& b, Block& 
 }
 
 // r -= a x
-template <class R, class X>
-__device__ __forceinline__ void subtract(const Block& a, const X& x, R& r) {
+__device__ __forceinline__ void subtract(const double (&a)[Q * Q], const double (&x)[Q], double (&r)[Q]) {
 #pragma unroll
   for (int i = 0; i < Q; ++i)
 #pragma unroll
@@ -124,11 +119,27 @@ __device__ __forceinline__ void from_lane(const Block& v, int src, Block& out) {
 
 // A lane's factors: its interior's, and per reduction level the multiples of the
 // rows `reach` lanes to the left and right that eliminate them.
-struct Factors {
-  lu_t lu[LU_SIZE];
-  Block left[LEVELS], right[LEVELS];  // the last level has one partner: left only
-  Block inverse;
+template <class T>
+struct FactorsOf {
+  T lu[LU_SIZE];
+  T left[LEVELS][Q * Q], right[LEVELS][Q * Q];  // the last level has one partner: left only
+  T inverse[Q * Q];
 };
+typedef FactorsOf<lu_t> Factors;    // as factorised
+typedef FactorsOf<double> Solver;   // as the stages solve with them
+
+__device__ __forceinline__ void widen(const Factors& F, Solver& S) {
+#pragma unroll
+  for (int i = 0; i < LU_SIZE; ++i) S.lu[i] = (double)F.lu[i];
+#pragma unroll
+  for (int i = 0; i < Q * Q; ++i) {
+#pragma unroll
+    for (int k = 0; k < LEVELS; ++k) S.left[k][i] = (double)F.left[k][i];
+#pragma unroll
+    for (int k = 0; k < LEVELS - 1; ++k) S.right[k][i] = (double)F.right[k][i];
+    S.inverse[i] = (double)F.inverse[i];
+  }
+}
 
 __device__ __forceinline__ int lane_at(const Lane& L, int offset) {
   return L.base + ((L.lane + offset) & (MDX_TEAM - 1));
@@ -191,11 +202,11 @@ __device__ __forceinline__ void factorize(Factors& F, const Block& next, const L
   invert(F.inverse);
 }
 
-__device__ __forceinline__ void solve(const Factors& F, lu_t (&r)[B], const Lane& L) {
-  lu_t left[Q], x[Q], xl[Q], xr[Q];
+__device__ __forceinline__ void solve(const Solver& F, double (&r)[B], const Lane& L) {
+  double left[Q], x[Q], xl[Q], xr[Q];
   if constexpr (HAS_INTERIOR) {
 #pragma unroll
-    for (int s = 0; s < Q; ++s) left[s] = (lu_t)0;
+    for (int s = 0; s < Q; ++s) left[s] = 0.0;
     interior_forward(F.lu, r, left);
   }
 #pragma unroll
@@ -220,7 +231,7 @@ __device__ __forceinline__ void solve(const Factors& F, lu_t (&r)[B], const Lane
   subtract(F.left[LEVELS - 1], xl, x);
 #pragma unroll
   for (int i = 0; i < Q; ++i) {
-    lu_t acc = F.inverse[i * Q] * x[0];
+    double acc = F.inverse[i * Q] * x[0];
 #pragma unroll
     for (int k = 1; k < Q; ++k) acc += F.inverse[i * Q + k] * x[k];
     r[separator(i)] = acc;
@@ -292,9 +303,9 @@ __device__ __forceinline__ bool running(const State& st, const MdxSolveArgs& a) 
 
 // Stage S: its right-hand side from f (in `work`) and the tableau row, then the solve.
 template <int S, class DT>
-__device__ __forceinline__ void stage(const Factors& F, k_t (&k)[8][B], const double (&work)[B], const DT& dT,
+__device__ __forceinline__ void stage(const Solver& F, double (&k)[8][B], const double (&work)[B], const DT& dT,
                                       double dt_use, double inv_dt, const Lane& L) {
-  lu_t r[B];
+  double r[B];
 #pragma unroll
   for (int j = 0; j < B; ++j) {
     double value = work[j];
@@ -304,25 +315,25 @@ __device__ __forceinline__ void stage(const Factors& F, k_t (&k)[8][B], const do
     (void)dt_use; (void)dT;
 #endif
     if constexpr (S > 0) {
-      double acc = coef_c(S, 0) * (double)k[0][j];
+      double acc = coef_c(S, 0) * k[0][j];
 #pragma unroll
-      for (int m = 1; m < S; ++m) acc += coef_c(S, m) * (double)k[m][j];
+      for (int m = 1; m < S; ++m) acc += coef_c(S, m) * k[m][j];
       value += acc * inv_dt;
     }
-    r[j] = (lu_t)value;
+    r[j] = value;
   }
   solve(F, r, L);
 #pragma unroll
-  for (int j = 0; j < B; ++j) k[S][j] = (k_t)r[j];
+  for (int j = 0; j < B; ++j) k[S][j] = r[j];
 }
 
 template <int S>
-__device__ __forceinline__ void advance(double (&u)[B], const State& st, const k_t (&k)[8][B]) {
+__device__ __forceinline__ void advance(double (&u)[B], const State& st, const double (&k)[8][B]) {
 #pragma unroll
   for (int j = 0; j < B; ++j) {
-    double acc = coef_a(S, 0) * (double)k[0][j];
+    double acc = coef_a(S, 0) * k[0][j];
 #pragma unroll
-    for (int m = 1; m <= S; ++m) acc += coef_a(S, m) * (double)k[m][j];
+    for (int m = 1; m <= S; ++m) acc += coef_a(S, m) * k[m][j];
     u[j] = st.y[j] + acc;
   }
 }
@@ -336,16 +347,18 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a, const Lan
   const double t_end = t + dt_use;
   const double inv_dt = recip_newton(dt_use);
 
-  Factors F;
+  Factors factors;
   Block next;
-  matrix(st.y, t, st.p, inv_dt * (1.0 / GAMMA), F.lu, next, L);
+  matrix(st.y, t, st.p, inv_dt * (1.0 / GAMMA), factors.lu, next, L);
   double dT[B];
 #if !MDX_AUTONOMOUS
   time_derivative(st.y, t, st.p, dT, L);
 #endif
-  factorize(F, next, L);
+  factorize(factors, next, L);
+  Solver F;
+  widen(factors, F);
 
-  k_t k[8][B];
+  double k[8][B];
   double u[B], work[B];
   rhs(st.y, t, st.p, work, L);
   stage<0>(F, k, work, dT, dt_use, inv_dt, L);
@@ -365,11 +378,11 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a, const Lan
   rhs(u, t_end, st.p, work, L);
   stage<5>(F, k, work, dT, dt_use, inv_dt, L);
 #pragma unroll
-  for (int j = 0; j < B; ++j) u[j] += (double)k[5][j];
+  for (int j = 0; j < B; ++j) u[j] += k[5][j];
   rhs(u, t_end, st.p, work, L);
   stage<6>(F, k, work, dT, dt_use, inv_dt, L);
 #pragma unroll
-  for (int j = 0; j < B; ++j) u[j] += (double)k[6][j];
+  for (int j = 0; j < B; ++j) u[j] += k[6][j];
   rhs(u, t_end, st.p, work, L);
   stage<7>(F, k, work, dT, dt_use, inv_dt, L);
 
@@ -378,7 +391,7 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a, const Lan
   double err = 0.0;
 #pragma unroll
   for (int j = 0; j < B; ++j) {
-    const double k7 = (double)k[7][j];
+    const double k7 = k[7][j];
     const double y_new = u[j] + k7;
     const double scale = a.atol + a.rtol * pymax(fabs(st.y[j]), fabs(y_new));
     const double r = weight(a, st.traj, L.lane * B + j) * k7 * recip_newton(scale);
@@ -409,17 +422,17 @@ __device__ __forceinline__ void step(State& st, const MdxSolveArgs& a, const Lan
       double* row = a.hist + hist_index(a, st.traj, st.save_idx, L);
 #pragma unroll
       for (int j = 0; j < B; ++j) {
-        double hsum = w[0] * (double)k[0][j];
+        double hsum = w[0] * k[0][j];
 #pragma unroll
-        for (int m = 1; m < 8; ++m) hsum += w[m] * (double)k[m][j];
-        const double y_new = u[j] + (double)k[7][j];
+        for (int m = 1; m < 8; ++m) hsum += w[m] * k[m][j];
+        const double y_new = u[j] + k[7][j];
         row[j] = theta1 * st.y[j] + theta * (y_new + theta1 * hsum);
       }
       ++st.save_idx;
       if (st.save_idx < a.n_save) st.next_save = a.times[st.save_idx];
     }
 #pragma unroll
-    for (int j = 0; j < B; ++j) st.y[j] = u[j] + (double)k[7][j];
+    for (int j = 0; j < B; ++j) st.y[j] = u[j] + k[7][j];
     st.t += dt_use;
     ++st.accepted;
   } else {
