@@ -131,7 +131,7 @@ def wide_solve_applies(options: KernelOptions) -> bool:
             and options.lu_precision == "fp32")
 
 
-# Dense systems up to this size invert their matrix in double by cofactors where they
+# Dense systems up to this size invert their matrix in closed form, in double, where they
 # would solve in double against FP32 factors (kernels/mdx_dense_lu.cuh, closed_inverse).
 CLOSED_INVERSE_MAX = 3
 

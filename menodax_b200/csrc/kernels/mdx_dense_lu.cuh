@@ -297,45 +297,98 @@ __device__ __forceinline__ void dense_solve_t_fast(const LU& lu, const IP& perm,
 }
 
 // --- systems of up to three states in fast arithmetic -------------------------------
-// The matrix is inverted in place in double by cofactors: one reciprocal, no pivot
-// search, and a solve is N independent rows of N multiply-adds instead of a
-// permutation and two substitutions, each row of which waits for the one before.
-// Its error is that of a double LU, so far below the FP32 factorisation's.  A
-// determinant past the double range would make a zero inverse, whose zero
-// increments pass any error test; it becomes NaN, which the controller rejects.
-// Robertson on a B200, whole calls, with the scaled system of mdx_rodas5p.cuh: 1
-// trajectory 218 -> 159 us, 8,191 from NumPy 482 -> 415, 65,536 524 -> 484.
+// The matrix is inverted in place in double: a solve is then N independent rows of N
+// multiply-adds instead of a permutation and two substitutions, each row of which waits
+// for the one before.  One and two states by cofactors, whose only cancellation is the
+// determinant's.  Cofactors of three states cancel twice: for one fast reaction
+// A + B <-> C, M = I + s u v^T, they are off by eps s^2 where an LU is by eps s, and at
+// s = 1e9 a solve took 15 times the steps.  So three states take one elimination step and
+// the cofactors of the two rows that remain, and lose what an LU does.  The remaining
+// rows are kept times the pivot: one reciprocal serves pivot and determinant, and all but
+// it and a multiply-add per entry is done while it is under way.  A determinant past the
+// double range would make a zero inverse, whose zero increments pass any error test; it
+// becomes NaN, which the controller rejects.
+//
+// The pivot is the first row's entry unless another's is over eight times as large, which
+// the exponents tell: rows in the order of an unconditional partial pivoting cost every
+// step 48 selects (3.5% of a solve).  Robertson on a B200, one launch, cofactors /
+// this: 1 trajectory 142 / 145 us, 65,536 370 / 374.  Pivoted LUs with FP32 factors in
+// place of both, and 1/h in the matrix (mdx_rodas5p.cuh), made the calls 218 and 524 us,
+// cofactors 159 and 484.
 constexpr int CLOSED_INVERSE_MAX = 3;
+
+__device__ __forceinline__ double inverse_or_nan(double det) { return finite(det) ? 1.0 / det : nan_value(); }
+
+// The exponent and leading 20 bits of |x|.
+__device__ __forceinline__ unsigned magnitude_word(double x) {
+  unsigned long long bits;
+  memcpy(&bits, &x, sizeof bits);
+  return (unsigned)(bits >> 32) & 0x7fffffffu;
+}
+
+__device__ __forceinline__ void swap_if(bool yes, double& a, double& b) {
+  const double c = yes ? b : a;
+  b = yes ? a : b;
+  a = c;
+}
+
+// The inverse of a 3 x 3 matrix with m[0] as the first pivot.
+template <class M, class X>
+__device__ __forceinline__ void inverse_by_first_pivot(const M& m, X& x) {
+  const double a = m[0];
+  // a times the rows that remain; their determinant is a times the matrix's.
+  const double s00 = a * m[4] - m[3] * m[1], s01 = a * m[5] - m[3] * m[2];
+  const double s10 = a * m[7] - m[6] * m[1], s11 = a * m[8] - m[6] * m[2];
+  const double det = s00 * s11 - s01 * s10;
+  const double q = inverse_or_nan(a * det);
+  const double left0 = s11 * m[3] - s01 * m[6], left1 = s00 * m[6] - s10 * m[3];
+  const double top0 = m[1] * s11 - m[2] * s10, top1 = m[2] * s00 - m[1] * s01;
+  const double corner = det + (m[1] * left0 + m[2] * left1);
+  const double r = a * q, ar = (a * a) * q;
+  x[0] = corner * q;
+  x[1] = -top0 * r;
+  x[2] = -top1 * r;
+  x[3] = -left0 * r;
+  x[4] = s11 * ar;
+  x[5] = -s01 * ar;
+  x[6] = -left1 * r;
+  x[7] = -s10 * ar;
+  x[8] = s00 * ar;
+}
 
 template <int N, class M>
 __device__ __forceinline__ void closed_inverse(M& m) {
-  static_assert(N <= CLOSED_INVERSE_MAX, "cofactors of up to three states");
-  double c[N * N];  // the adjugate
-  double det;
+  static_assert(N <= CLOSED_INVERSE_MAX, "closed forms of up to three states");
   if constexpr (N == 1) {
-    c[0] = 1.0;
-    det = m[0];
+    m[0] = inverse_or_nan(m[0]);
   } else if constexpr (N == 2) {
-    c[0] = m[3];
-    c[1] = -m[1];
-    c[2] = -m[2];
-    c[3] = m[0];
-    det = m[0] * m[3] - m[1] * m[2];
+    const double r = inverse_or_nan(m[0] * m[3] - m[1] * m[2]);
+    const double first = m[0];
+    m[0] = m[3] * r;
+    m[1] = -m[1] * r;
+    m[2] = -m[2] * r;
+    m[3] = first * r;
   } else {
-    c[0] = m[4] * m[8] - m[5] * m[7];
-    c[1] = m[2] * m[7] - m[1] * m[8];
-    c[2] = m[1] * m[5] - m[2] * m[4];
-    c[3] = m[5] * m[6] - m[3] * m[8];
-    c[4] = m[0] * m[8] - m[2] * m[6];
-    c[5] = m[2] * m[3] - m[0] * m[5];
-    c[6] = m[3] * m[7] - m[4] * m[6];
-    c[7] = m[1] * m[6] - m[0] * m[7];
-    c[8] = m[0] * m[4] - m[1] * m[3];
-    det = m[0] * c[0] + (m[1] * c[3] + m[2] * c[6]);
-  }
-  const double r = finite(det) ? 1.0 / det : nan_value();
+    double x[N * N];
+    inverse_by_first_pivot(m, x);
+    const unsigned w0 = magnitude_word(m[0]), w1 = magnitude_word(m[3]), w2 = magnitude_word(m[6]);
+    if ((w1 > w2 ? w1 : w2) > w0 + (3u << 20)) {  // 2^3 times m[0]
+      // The largest entry's row first; the inverse's columns go back the same way.
+      const bool second = fabs(m[3]) > fabs(m[0]);
 #pragma unroll
-  for (int i = 0; i < N * N; ++i) m[i] = c[i] * r;
+      for (int j = 0; j < 3; ++j) swap_if(second, m[j], m[3 + j]);
+      const bool third = fabs(m[6]) > fabs(m[0]);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) swap_if(third, m[j], m[6 + j]);
+      inverse_by_first_pivot(m, x);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) swap_if(third, x[3 * i], x[3 * i + 2]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) swap_if(second, x[3 * i], x[3 * i + 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < N * N; ++i) m[i] = x[i];
+  }
 }
 
 // x = M^-1 b and (TRANSPOSED) x = M^-T b, in place.

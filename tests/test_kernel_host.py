@@ -426,3 +426,25 @@ def test_rodas5p_time_derivative_and_tf_index(tmp_path):
     stops = int(np.searchsorted(t_span, 0.5, side="right"))
     np.testing.assert_allclose(hist[1, :stops, 0], exact[:stops], rtol=1e-8, atol=1e-10)
     assert (hist[1, stops:, 0] == hist[1, stops - 1, 0]).all()
+
+
+@pytest.mark.parametrize("rate", [1e7, 1e9])
+def test_one_fast_reaction_takes_the_steps_of_a_double_lu(tmp_path, rate):
+    """A + B <-> C with a slow drain: one fast mode that couples all three states.  The
+    default solve inverts its matrix in closed form; an inverse less accurate than an LU's
+    shows as rejected steps (two and fifteen times the steps at these rates)."""
+    def fn(y, t, p):
+        net = rate * y[0] * y[1] - p[0] * rate * y[2]
+        return -net + 0.1 - 0.1 * y[0], -net + 0.05 - 0.1 * y[1], net - 0.1 * y[2]
+
+    y0 = np.random.default_rng(3).uniform(0.2, 1.0, (8, 3))
+    params, times = np.linspace(0.05, 0.5, 8)[:, None], np.linspace(0.0, 50.0, 6)
+    runs = {}
+    for name, options in (("closed", KernelOptions(lu_precision="fp32", fast=True)),
+                          ("lu", KernelOptions(lu_precision="fp64", fast=True))):
+        lib = _host_kernel(tmp_path, name, fn, 3, 1, options)
+        runs[name] = _solve(lib, y0, times, params, 1e-6, 1e-10)
+    (h, c), (h0, c0) = runs["closed"], runs["lu"]
+    assert (c[3] == 0).all()
+    assert c[2].mean() <= 1.05 * c0[2].mean() + 1
+    np.testing.assert_allclose(h, h0, rtol=2e-5, atol=1e-9)

@@ -107,9 +107,10 @@ CLOSED(1) CLOSED(2) CLOSED(3)
 
 @pytest.mark.parametrize("n", [1, 2, 3])
 def test_closed_inverse(tmp_path, n):
-    """Cofactors against NumPy: each entry is a few products, so the inverse is off by at
-    most about 8 n roundings times the condition number; a determinant past the range of a
-    double gives NaN, not the zero that would pass an error test."""
+    """Row-scaled random matrices against NumPy: an entry is a few products over the
+    determinant, so the inverse is off by at most about 8 n roundings times the condition number;
+    a determinant past the range of a double gives NaN, not the zero that would pass an error
+    test."""
     (tmp_path / "c.cpp").write_text(PRELUDE + CLOSED)
     subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", f"-I{KERNEL_DIR}", str(tmp_path / "c.cpp"),
                     "-o", str(tmp_path / "c.so")], check=True)
@@ -126,3 +127,46 @@ def test_closed_inverse(tmp_path, n):
         assert np.linalg.norm(xt - np.linalg.solve(a.T, b)) <= bound
     run(_p(np.eye(n) * 1e200 if n > 1 else np.array([[np.inf]])), _p(np.ones(n)), _p(x), _p(xt))
     assert np.isnan(x).all()
+
+
+@pytest.mark.parametrize("modes", [1, 2])
+def test_closed_inverse_of_fast_modes_is_as_accurate_as_an_lu(tmp_path, lib, modes):
+    """M = I + s u v^T (one fast reaction that couples all three states, and a second at
+    sqrt(s)), in states of very different sizes: an LU loses eps s of a solve, cofactors of the
+    whole matrix eps s^2.  The two orders of elimination round differently, by less than a
+    factor of four in the median of 50."""
+    from fractions import Fraction
+
+    (tmp_path / "c.cpp").write_text(PRELUDE + CLOSED)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC", "-w", f"-I{KERNEL_DIR}",
+                    str(tmp_path / "c.cpp"), "-o", str(tmp_path / "c.so")], check=True)
+    run = ctypes.CDLL(str(tmp_path / "c.so")).closed3
+    rng = np.random.default_rng(modes)
+
+    def exact(m, b):  # Cramer's rule in rational numbers
+        m = [[Fraction(v) for v in row] for row in m]
+        det = lambda a: (a[0][0] * (a[1][1] * a[2][2] - a[1][2] * a[2][1])  # noqa: E731
+                         - a[0][1] * (a[1][0] * a[2][2] - a[1][2] * a[2][0])
+                         + a[0][2] * (a[1][0] * a[2][1] - a[1][1] * a[2][0]))
+        whole = det(m)
+        return np.array([float(det([[Fraction(b[i]) if k == j else m[i][k] for k in range(3)] for i in range(3)]) / whole)
+                         for j in range(3)])
+
+    for s in 10.0 ** np.arange(0, 11):
+        errors = []
+        for _ in range(50):
+            m = np.eye(3)
+            for size in (s, np.sqrt(s))[:modes]:
+                u, v = rng.normal(size=(2, 3))
+                m += size * np.outer(u, v if u @ v > 0 else -v)
+            scale = np.exp(rng.uniform(-10, 10, 3))
+            m *= scale[None, :] / scale[:, None]
+            b, x, xt, y, yt = rng.normal(size=3), *np.empty((4, 3))
+            run(_p(m), _p(b), _p(x), _p(xt))
+            lib.solve_double3(_p(m), _p(b), _p(y), 0, 0)
+            lib.solve_double3(_p(m), _p(b), _p(yt), 1, 0)
+            right, right_t = exact(m, b), exact(m.T, b)
+            errors.append([np.linalg.norm(got - ref) / np.linalg.norm(ref)
+                           for got, ref in ((x, right), (y, right), (xt, right_t), (yt, right_t))])
+        closed, lu, closed_t, lu_t = np.median(errors, axis=0)
+        assert closed <= 4 * max(lu, 2.0 ** -53) and closed_t <= 4 * max(lu_t, 2.0 ** -53), s
