@@ -37,7 +37,8 @@ launch, since long stiff ensembles have uneven step counts.  The cost of a step
 does not see the longest trajectories' tail, which more lanes shorten and an order
 by what remains after the first steps (a staged launch) takes from the end: the
 winner's persistent launch, the cyclic kernel's and the staged form of the fastest
-are timed in full, while that fits ``BUDGET_S``.
+are timed in full, where runs under longer and longer caps show that this fits
+``BUDGET_S``; otherwise the capped run decides.
 """
 
 from __future__ import annotations
@@ -67,6 +68,7 @@ BLOCK_SIZES = (32, 64, 128)
 PERSISTENT_FILL = (1.0, 0.5)
 PROBE = 4096
 PROBE_STEPS = 500
+CAP_GROWTH = 4   # between the caps that find how long whole integrations take
 BUDGET_S = 3.0
 TEAM_MIN_VARS = 16
 SHARED_STAGES_MAX_VARS = 16   # the reference's bound for its shared Tsit5 backend
@@ -225,26 +227,43 @@ def _timed_sort(steps, stream) -> float:
     return e0.elapsed_time(e1) * 1e-3
 
 
-def _fastest_in_full(problem_for, stream, n, max_steps, inputs, choice, buildable):
+def _fastest_in_full(problem_for, stream, n, max_steps, inputs, choice, buildable, capped_s):
     """``choice`` or the cyclic persistent launch that finishes the whole ensemble first, in
-    its staged form where that is at least ``STAGE_GAIN`` faster still; stops timing once the
-    launches so far have taken ``BUDGET_S``."""
+    its staged form where that is at least ``STAGE_GAIN`` faster still; ``choice`` where
+    finding that out would take over ``BUDGET_S``.
+
+    ``capped_s`` holds the plain launches' seconds under ``PROBE_STEPS``.  How long a whole
+    integration takes is found by raising the cap ``CAP_GROWTH``-fold until every trajectory
+    ends below it, each run only if it fits the budget at the last one's cost a step."""
     spent = 0.0
 
-    def timed(candidate):
+    def timed(candidate, cap):
         nonlocal spent
-        secs, _ = _timed_launch(problem_for(candidate), candidate, stream, n=n, max_steps=max_steps, **inputs)
+        secs, counters = _timed_launch(problem_for(candidate), candidate, stream, n=n, max_steps=cap, **inputs)
         spent += secs
-        return secs
+        return secs, counters
 
-    best = timed(choice), choice
+    def capped(candidate):
+        return capped_s[replace(candidate, mode=_native.MDX_LAUNCH_PLAIN, grid_fill=0.0)]
+
+    cap, secs, ended = PROBE_STEPS, capped(choice), False
+    while not ended:
+        if spent + CAP_GROWTH * secs > BUDGET_S:
+            return choice
+        cap = min(int(max_steps), CAP_GROWTH * cap)
+        secs, counters = timed(choice, cap)
+        ended = cap == int(max_steps) or int(counters[2].max()) < cap
+    best, whole = (secs, choice), secs
     for candidate in buildable:
-        if (candidate.cyclic and candidate.mode == _native.MDX_LAUNCH_PERSISTENT and candidate != choice
-                and spent + best[0] <= BUDGET_S):
-            best = min(best, (timed(candidate), candidate), key=lambda timing: timing[0])
-    if (best[1].cyclic or not best[1].team) and spent + best[0] <= BUDGET_S:
+        if not candidate.cyclic or candidate.mode != _native.MDX_LAUNCH_PERSISTENT or candidate == choice:
+            continue
+        if spent + whole * max(1.0, capped(candidate) / capped(choice)) <= BUDGET_S:
+            best = min(best, (timed(candidate, cap)[0], candidate), key=lambda timing: timing[0])
+    if (best[1].cyclic or not best[1].team) and spent + 3 * best[0] <= BUDGET_S:
         staged = replace(best[1], staged=True)
-        if timed(staged) <= (1.0 - STAGE_GAIN) * best[0]:
+        first = timed(staged, cap)[0]
+        unstaged_s = min(best[0], timed(best[1], cap)[0])
+        if min(first, timed(staged, cap)[0]) <= (1.0 - STAGE_GAIN) * unstaged_s:
             return staged
     return best[1]
 
@@ -392,16 +411,14 @@ def _tuned(call, *, y0, times, params, weights, dt0, rtol, atol, n_save_hist):
     probe_s, counters = _timed_launch(problem_for(first), first, stream, n=n, max_steps=cap, **inputs)
     capped = cap < int(max_steps) and int(counters[2].max()) >= cap
     if capped:
-        best = None
+        capped_s = {}
         for choice in buildable:
             if choice.mode != _native.MDX_LAUNCH_PLAIN:
                 continue
             prob = problem_for(choice)
             _timed_launch(prob, choice, stream, n=n, max_steps=cap, **inputs)
-            secs, _ = _timed_launch(prob, choice, stream, n=n, max_steps=cap, **inputs)
-            if best is None or secs < best[0]:
-                best = (secs, choice)
-        winner = best[1]
+            capped_s[choice], _ = _timed_launch(prob, choice, stream, n=n, max_steps=cap, **inputs)
+        winner = min(capped_s, key=capped_s.get)
         fill = 1.0 if winner.team else 0.5
         persistent = [c for c in buildable if c.mode == _native.MDX_LAUNCH_PERSISTENT and c.team == winner.team
                       and c.threads_per_block == winner.threads_per_block and c.grid_fill == fill
@@ -409,7 +426,7 @@ def _tuned(call, *, y0, times, params, weights, dt0, rtol, atol, n_save_hist):
                       and c.cyclic == winner.cyclic and c.inverse == winner.inverse]
         choice = persistent[0] if persistent else winner
         if tune_registers and choice.mode == _native.MDX_LAUNCH_PERSISTENT:
-            choice = _fastest_in_full(problem_for, stream, n, max_steps, inputs, choice, buildable)
+            choice = _fastest_in_full(problem_for, stream, n, max_steps, inputs, choice, buildable, capped_s)
         with _lock:
             _cache[key] = choice
         return choice

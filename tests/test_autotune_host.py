@@ -193,3 +193,26 @@ def test_host_results_of_short_persistent_thread_launches_stream_from_the_one_la
     assert not autotune.streams_to_host(autotune.LaunchChoice(128, PERSISTENT, 0.5, 0))
     assert not autotune.streams_to_host(autotune.LaunchChoice(128, PERSISTENT, 1.0, 8))
     assert not autotune.streams_to_host(autotune.LaunchChoice(128, PLAIN, 0.0, 0))
+
+
+@pytest.mark.parametrize("whole_s,timed_in_full", [(20.0, False), (0.2, True)])
+def test_whole_integrations_are_timed_only_within_the_budget(fake_device, monkeypatch, whole_s, timed_in_full):
+    """Launches that take ``whole_s`` uncapped, at an even cost a step.  Where one would take
+    longer than the budget none runs uncapped, and the runs that find this out stay within
+    the budget; where it is short, the staged form is timed beside it, twice each."""
+    fn, n, pattern = _ring(16)
+    opts = KernelOptions(lu_precision="fp32", fast=True, sparsity=pattern)
+
+    def cost(choice, n_traj, steps):
+        return whole_s * steps / 100000 * (0.9 if choice.staged else 1.0) * (1.0 if choice.team == 8 else 1.2)
+
+    rec = Recorder(cost, steps=100000)
+    choice = _tune(fn, n, opts, rec, monkeypatch, tune_team=True, tune_registers=True)
+    assert (choice.team, choice.cyclic, choice.mode, choice.staged) == (8, True, PERSISTENT, timed_in_full)
+    beyond = [(c, s) for c, _, s in rec.calls if s > autotune.PROBE_STEPS]
+    assert sum(cost(c, 0, s) for c, s in beyond) <= autotune.BUDGET_S
+    full = [c for c, s in beyond if s == 100000]
+    if timed_in_full:
+        assert sum(c.staged for c in full) == 2 and {c.team for c in full} == {4, 8, 16}
+    else:
+        assert not full
