@@ -108,7 +108,7 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
 
         choice = autotune.tune(ode_fn, n_vars, n_params, options, tune_block=tune_block,
                                tune_team=tune_team, tune_shared=tune_shared, tune_registers=tune_team,
-                               tune_orders=True, **common)
+                               tune_orders=True, span=None if times.is_cuda else float(times[-1] - times[0]), **common)
         options = autotune.options_for(options, choice)
         problem = get_problem(ode_fn, n_vars, n_params, options)
         mode = choice.mode

@@ -92,6 +92,7 @@ class LaunchChoice:
     cyclic: bool = False  # with a team: the cyclic kernel, a block of the state per lane
     inverse: bool = False  # with a team, dense: M inverted in registers
     staged: bool = False   # persistent: every trajectory's first steps, then the rest longest first
+    staged_length: float = 0.0  # the integration_length over which staging was measured to gain
 
     def describe(self) -> str:
         kind = "plain" if self.mode == _native.MDX_LAUNCH_PLAIN else f"{'staged' if self.staged else 'persistent'}(fill={self.grid_fill})"
@@ -164,6 +165,12 @@ STAGE_STEPS = 128
 # 29.6 ms, [0, 3000] 287 / 253 (ordered by exact step counts 249); 32 states on cyclic
 # lanes, whose longest trajectories set the time in any order, 22.9 / 23.2.
 STAGE_GAIN = 0.03
+
+
+def integration_length(span: float, rtol: float) -> float:
+    """What the step count of an integration grows with: its span, and rtol^(-1/6) for a
+    method whose local error is of sixth order in the step."""
+    return abs(span) * max(rtol, 1e-16) ** (-1.0 / 6.0)
 
 
 def slice_steps(choice: LaunchChoice) -> int:
@@ -310,7 +317,7 @@ def _spread(lanes, n: int) -> int:
 
 def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, rtol, atol,
          max_steps, n_save_hist=None, tune_block=True, tune_team=False, tune_shared=False,
-         tune_registers=False, tune_orders=False):
+         tune_registers=False, tune_orders=False, span=None):
     """The fastest launch for this problem on these inputs (device tensors).
 
     With ``tune_block=False`` the block size stays ``options.threads_per_block``
@@ -327,6 +334,9 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
     With ``tune_shared`` (Tsit5) the launches with the stage vectors in shared
     memory are candidates beside the register ones; ``options.shared_stages``
     already set keeps them there.
+    ``span`` is the integration's, where the caller knows it without asking the device: a
+    staged launch is for integrations at least half as long (``integration_length``) as the one
+    it was measured on, and the same launch unstaged for shorter ones.
 
     The first candidate runs once on the whole ensemble with at most
     ``PROBE_STEPS`` steps per trajectory.  If that finished every trajectory, its
@@ -342,11 +352,16 @@ def tune(ode_fn, n_vars, n_params, options, *, y0, times, params, weights, dt0, 
             tune_orders)
     with _lock:
         found = _cache.get(call)
+    length = None if span is None else integration_length(span, rtol)
     if found is None:
         found = _tuned(call, y0=y0, times=times, params=params, weights=weights, dt0=dt0, rtol=rtol, atol=atol,
                        n_save_hist=n_save_hist)
+        if found.staged:
+            found = replace(found, staged_length=length or 0.0)
         with _lock:
             _cache[call] = found
+    if found.staged and length is not None and length < 0.5 * found.staged_length:
+        return replace(found, staged=False)
     return found
 
 
@@ -384,7 +399,7 @@ def _tuned(call, *, y0, times, params, weights, dt0, rtol, atol, n_save_hist):
         solves = (False, True)
     cands = candidates(blocks, teams, shared_blocks, options.shared_stages, solves, cyclic, inverse)
     key = (ode_fn, n_vars, n_params, replace(options, threads_per_block=32, team=0, shared_stages=False), n,
-           tuple(cands), max_steps, torch.cuda.get_device_name(y0.device), tune_orders)
+           tuple(cands), max_steps, torch.cuda.get_device_name(y0.device), tune_registers, tune_orders)
     with _lock:
         found = _cache.get(key)
     if found is not None:

@@ -216,3 +216,25 @@ def test_whole_integrations_are_timed_only_within_the_budget(fake_device, monkey
         assert sum(c.staged for c in full) == 2 and {c.team for c in full} == {4, 8, 16}
     else:
         assert not full
+
+
+def test_short_integrations_do_not_take_a_staged_choice_of_long_ones(fake_device, monkeypatch):
+    """Equal ensembles share a tuned launch, but not its staging over integrations far
+    shorter than the measured one, by span or by tolerance."""
+    fn, n, pattern = _ring(16)
+    opts = KernelOptions(lu_precision="fp32", fast=True, sparsity=pattern)
+    rec = Recorder(lambda c, m, s: 0.1 * (0.9 if c.staged else 1.0), steps=100000)
+    long = _tune(fn, n, opts, rec, monkeypatch, tune_team=True, tune_registers=True, span=300.0)
+    assert long.staged
+    count = len(rec.calls)
+    for span, staged in ((300.0, True), (200.0, True), (100.0, False), (1.0, False), (None, True)):
+        choice = _tune(fn, n, opts, rec, monkeypatch, tune_team=True, tune_registers=True, span=span)
+        assert choice.staged == staged and (choice.team, choice.mode) == (long.team, long.mode)
+    assert len(rec.calls) == count                       # none of them is tuned again
+    assert autotune.integration_length(300.0, 1e-3) < 0.5 * long.staged_length
+
+    # Nor does a caller that cannot stage find the choice of one that can.
+    fn, n, pattern = _ring(4)
+    opts = KernelOptions(lu_precision="fp32", fast=True, sparsity=pattern)
+    assert _tune(fn, n, opts, rec, monkeypatch, tune_registers=True).staged
+    assert not _tune(fn, n, opts, rec, monkeypatch).staged
