@@ -61,8 +61,9 @@ def _times_tensor(t_span):
     return t
 
 
-# Below this many trajectories a launch is one partial wave whatever its shape,
-# and the reference's own choice (one warp per block, one launch) is kept.
+# Below this many trajectories a launch is one partial wave whatever its shape, so
+# nothing is timed: one launch, of one warp per block (the reference's own choice) or, for
+# systems that gain from more lanes a trajectory, of autotune.small_choice's.
 AUTOTUNE_MIN_TRAJECTORIES = 4096
 
 

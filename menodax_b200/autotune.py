@@ -62,6 +62,7 @@ from menodax_b200._problem import (
     tsit5_stage_bytes,
     wide_solve_applies,
 )
+from menodax_b200._sparse_direct import sparse_lu_for
 from menodax_b200._team import TEAM_SIZES
 
 BLOCK_SIZES = (32, 64, 128)
@@ -283,10 +284,10 @@ def small_choice(ode_fn, n_vars, n_params, options, n) -> LaunchChoice | None:
     trajectories on a B200, 4 / 8 / 16 / 32 lanes: the 32-state ring 25.2 / 19.3 / 15.3
     ms / --, the 64-state Brusselator -- / 0.90 / 0.65 / 0.51 ms; on the shared-memory teams
     64.4 and 3.5 ms, on threads slower still).  Other systems of ``TEAM_MIN_VARS`` states or
-    more take a team by the same rule: a thread's vectors no longer fit its registers, nor a
-    dense matrix at all (256 trajectories: dense 32 states 94.6 ms on threads, 4.2 on
-    32-lane teams, 1.0 with the register inverse; sparse 64 states 0.75 on threads, 0.18 on
-    32 lanes)."""
+    more take a team by the same rule where it gains.  Dense ones all do: a thread's matrix no
+    longer fits its registers (256 trajectories, 32 states: 94.6 ms on threads, 4.2 on 32-lane
+    teams, 1.0 with the register inverse; at 16 to 40 states, 1 to 4,095 trajectories and any
+    precision 1.75 to 75 times as fast).  Sparse ones: ``_sparse_team_gains``."""
     lanes = cyclic_lanes(ode_fn, n_vars, n_params, options)
     if lanes:
         return LaunchChoice(CYCLIC_BLOCK, _native.MDX_LAUNCH_PLAIN, 0.0, _spread(lanes, n), cyclic=True)
@@ -305,8 +306,34 @@ def small_choice(ode_fn, n_vars, n_params, options, n) -> LaunchChoice | None:
     # 256 trajectories 1.02 / 1.75 ms, 1,500 1.63 / 2.28, 4,097 3.79 / 4.77.
     widest = max(teams)
     team = widest if team_inverse_fits(n_vars, replace(options, team=widest)) else _spread(teams, n)
+    if options.sparsity is not None and not _sparse_team_gains(n_vars, options, team):
+        return None
     return LaunchChoice(32, _native.MDX_LAUNCH_PLAIN, 0.0, team,
                         inverse=team_inverse_fits(n_vars, replace(options, team=team)))
+
+
+def _sparse_team_gains(n_vars: int, options, team: int) -> bool:
+    """Whether a small ensemble of a sparse system is faster on ``team`` lanes a trajectory
+    than on one.
+
+    A team shares the vectors, but its first lane factorises and solves alone, out of shared
+    memory instead of a thread's registers: the more of a step the LU is (its entries a state),
+    the larger the system that gains.  Threads over teams, 1 to 4,095 trajectories on a B200:
+
+    - 16 states: tridiagonal, 3 entries a state, 1.05 to 1.3 on 16 lanes, 0.77 to 0.90 on 8;
+      4.6 to 10 entries 0.56 to 0.97 on any.
+    - 24 to 31 states: 3 entries 1.1 to 2.8 on 16 and 32 lanes, on 8 in FP32 1.07 to 1.5 and in
+      FP64 0.91 to 1.2; 5 to 8 entries 1.1 to 1.6 on 8 and 16 lanes, 0.89 to 1.2 on 32; 13
+      entries 0.79 to 1.06.
+    - 32 states and more: up to 10 entries 0.98 to 6.8; 15 to 18 entries in FP32 0.94 to 1.1 at 32
+      states, 1.04 to 1.8 from 36, in FP64 1.2 to 2.0 on 32 lanes and 0.66 to 1.2 on fewer."""
+    entries = sparse_lu_for(options.sparsity, options.ordering).slots.size / n_vars
+    fp32 = options.lu_precision == "fp32"
+    if n_vars < 24:
+        return entries <= 3 and team >= 16
+    if n_vars < 32:
+        return (team >= 16 or fp32) if entries <= 3 else entries <= 8 and team <= 16
+    return entries <= 12 or (n_vars >= 36 if fp32 else team == 32)
 
 
 def _spread(lanes, n: int) -> int:

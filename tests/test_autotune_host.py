@@ -238,3 +238,27 @@ def test_short_integrations_do_not_take_a_staged_choice_of_long_ones(fake_device
     opts = KernelOptions(lu_precision="fp32", fast=True, sparsity=pattern)
     assert _tune(fn, n, opts, rec, monkeypatch, tune_registers=True).staged
     assert not _tune(fn, n, opts, rec, monkeypatch).staged
+
+
+def _banded(n, width):
+    return tuple(tuple(range(max(0, i - width), min(n, i + width + 1))) for i in range(n))
+
+
+@pytest.mark.parametrize("n_vars,width,lu,size,on_a_team", [
+    (16, 1, "fp32", 300, True), (16, 1, "fp32", 4095, False),     # 8 lanes are too few
+    (16, 2, "fp32", 300, False), (16, 15, "fp64", 1, False),      # the LU runs on one lane
+    (24, 1, "fp64", 300, True), (24, 1, "fp64", 4095, False), (24, 1, "fp32", 4095, True),
+    (24, 2, "fp32", 300, False), (24, 2, "fp32", 1500, True), (24, 23, "fp32", 1500, False),
+    (32, 3, "fp64", 1, True), (32, 31, "fp32", 300, False), (36, 35, "fp32", 4095, True),
+    (48, 47, "fp64", 300, True), (48, 47, "fp64", 1500, False),
+])
+def test_small_sparse_ensembles_take_a_team_where_it_was_measured_to_gain(n_vars, width, lu, size, on_a_team):
+    """A system that does not repeat around a ring (its ends differ)."""
+    fn, _ = systems.make_heat_system(n_vars)
+    options = KernelOptions(lu_precision=lu, fast=lu == "fp32", sparsity=_banded(n_vars, width))
+    choice = autotune.small_choice(fn, n_vars, 1, options, size)
+    assert (choice is not None) == on_a_team
+    if on_a_team:
+        assert choice.team and not choice.cyclic and choice.mode == PLAIN
+    dense = autotune.small_choice(fn, n_vars, 1, KernelOptions(lu_precision=lu, fast=lu == "fp32"), size)
+    assert dense is not None and dense.team
