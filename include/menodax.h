@@ -239,6 +239,11 @@ int mdx_sens_contract(const double* joint, const double* cotangent, int n_traj, 
  * counterpart in the reference. */
 int mdx_measure_fma_peak(int double_precision, double* flops_per_s);
 
+/* *yes = 1 where pageable host memory goes to `device` through the driver's own page-locked
+ * memory, so that an asynchronous copy from it has read it when the call returns; 0 where
+ * the device reads it through the host's page tables, whenever the copy runs. */
+int mdx_stages_pageable_copies(int device, int* yes);
+
 /* The calling thread's last error message. Returns its full length. */
 int mdx_last_error(char* buf, size_t buf_size);
 

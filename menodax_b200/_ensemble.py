@@ -7,6 +7,8 @@ call and the stats dict), with torch providing device memory and the stream.
 
 from __future__ import annotations
 
+from functools import lru_cache
+
 import numpy as np
 import torch
 
@@ -107,7 +109,8 @@ def to_device(t, device):
     memory by the time an asynchronous copy from it returns, so the caller may change or free it
     at once (page-locked memory it reads later, as it did before).  A waiting copy of the save
     times alone (160 bytes) made each solve wait for the one before: 100 us of a 200 us call
-    on a B200.  During a stream capture the copy waits, which the capture refuses, rather than
+    on a B200.  Where the driver says that a device reads pageable memory itself
+    (``mdx_stages_pageable_copies``) the copy waits.  During a stream capture the copy waits, which the capture refuses, rather than
     become a node that reads host memory at replay."""
     if t is None:
         return None
@@ -115,8 +118,14 @@ def to_device(t, device):
         return t
     if t.is_cuda or device.type != "cuda":
         return t.to(device=device).contiguous()
-    waits = not t.is_pinned() and torch.cuda.is_current_stream_capturing()
-    return t.contiguous().to(device=device, non_blocking=not waits)
+    t = t.contiguous()  # a copy of a page-locked tensor is pageable, and gone after this call
+    waits = not t.is_pinned() and (torch.cuda.is_current_stream_capturing() or not _staged_copies(device.index))
+    return t.to(device=device, non_blocking=not waits)
+
+
+@lru_cache(maxsize=None)
+def _staged_copies(index) -> bool:
+    return _native.stages_pageable_copies(torch.cuda.current_device() if index is None else index)
 
 
 class Workspace:

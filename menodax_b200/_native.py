@@ -46,6 +46,7 @@ EXPORTED = (
     "mdx_measure_fma_peak", "mdx_solve_persistent_noalloc", "mdx_checkpoint_size",
     "mdx_order_workspace_size", "mdx_order_longest_first",
     "mdx_sens_contract", "mdx_staged_workspace_size", "mdx_solve_staged",
+    "mdx_stages_pageable_copies",
 )
 
 
@@ -158,6 +159,7 @@ def lib():
         L.mdx_staged_workspace_size.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_size_t)]
         L.mdx_solve_staged.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveDesc), ctypes.c_int, ctypes.c_void_p,
                                        ctypes.c_size_t, ctypes.c_void_p]
+        L.mdx_stages_pageable_copies.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
         L.mdx_measure_fma_peak.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
         _lib = L
         return _lib
@@ -168,6 +170,14 @@ def measure_fma_peak(double_precision: bool = True) -> float:
     out = ctypes.c_double()
     check(lib().mdx_measure_fma_peak(1 if double_precision else 0, ctypes.byref(out)), "mdx_measure_fma_peak")
     return out.value
+
+
+def stages_pageable_copies(device: int) -> bool:
+    """Whether the driver copies pageable host memory through page-locked memory of its own
+    on the way to ``device``, and so has read it when an asynchronous copy returns."""
+    out = ctypes.c_int()
+    check(lib().mdx_stages_pageable_copies(device, ctypes.byref(out)), "mdx_stages_pageable_copies")
+    return bool(out.value)
 
 
 def order_workspace_size() -> int:

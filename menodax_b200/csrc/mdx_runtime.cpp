@@ -610,6 +610,19 @@ StageLayout stage_layout(const mdx_plan* plan, int n_traj) {
 
 extern "C" {
 
+int mdx_stages_pageable_copies(int device, int* yes) {
+  if (!yes) return fail(MDX_E_INVALID, "mdx_stages_pageable_copies: null argument");
+  if (int rc = require_driver()) return rc;
+  CUdevice dev;
+  CUresult r = g_driver.deviceGet(&dev, device);
+  if (r != CUDA_SUCCESS) return cuda_fail(r, "cuDeviceGet");
+  int direct = 0;
+  r = g_driver.deviceGetAttribute(&direct, CU_DEVICE_ATTRIBUTE_PAGEABLE_MEMORY_ACCESS_USES_HOST_PAGE_TABLES, dev);
+  if (r != CUDA_SUCCESS) return cuda_fail(r, "cuDeviceGetAttribute");
+  *yes = direct ? 0 : 1;
+  return MDX_OK;
+}
+
 int mdx_staged_workspace_size(const mdx_plan* plan, int n_traj, size_t* bytes) {
   if (!plan || !bytes) return fail(MDX_E_INVALID, "mdx_staged_workspace_size: null argument");
   if (n_traj < 0) return fail(MDX_E_INVALID, "n_traj must be non-negative");

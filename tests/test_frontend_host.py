@@ -65,3 +65,45 @@ def test_a_half_filled_persistent_launch_is_kept_and_copied_after_the_kernel(stu
     second = stub_device[-1]
     assert second["order"] is not None and second["order"].dtype == torch.int32
     assert second["order"].numel() == 4096
+
+
+class HostTensor:
+    """What ``to_device`` asks of a host tensor, and the copies it starts."""
+
+    device, is_cuda = torch.device("cpu"), False
+
+    def __init__(self, copies, pinned=False, dense=True):
+        self.copies, self.pinned, self.dense = copies, pinned, dense
+
+    def is_contiguous(self):
+        return self.dense
+
+    def contiguous(self):
+        return self if self.dense else HostTensor(self.copies)
+
+    def is_pinned(self):
+        return self.pinned
+
+    def to(self, *, device, non_blocking):
+        self.copies.append((self.pinned, non_blocking))
+        return self
+
+
+@pytest.mark.parametrize("staged", [True, False])
+@pytest.mark.parametrize("capturing", [True, False])
+def test_host_copies_wait_where_the_driver_may_read_them_later(monkeypatch, staged, capturing):
+    """An asynchronous copy from pageable memory only where the driver has read it on return:
+    not on devices that read it themselves, not as a node of a graph, and a page-locked
+    tensor's contiguous copy is pageable too."""
+    from menodax_b200 import _ensemble
+
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+    monkeypatch.setattr(_native, "stages_pageable_copies", lambda device: staged)
+    _ensemble._staged_copies.cache_clear()
+    copies = []
+    for pinned in (False, True):
+        for dense in (False, True):
+            _ensemble.to_device(HostTensor(copies, pinned, dense), torch.device("cuda", 0))
+    _ensemble._staged_copies.cache_clear()
+    free = staged and not capturing
+    assert copies == [(False, free), (False, free), (False, free), (True, True)]

@@ -190,3 +190,27 @@ def test_registered_host_memory_and_refusals():
     # The Python launcher checks the tensor before the runtime sees it.
     with pytest.raises(ValueError, match="hist_host"):
         launch(problem, hist_host=torch.empty((n, s, 3), dtype=torch.float64), **args)
+
+
+def test_pageable_inputs_may_change_as_soon_as_the_call_returns():
+    """Their copies do not wait for the stream: with the stream held up for some tens of
+    milliseconds the solve returns before anything has run, and the caller overwrites what it
+    passed (save times, and an initial state large enough for several staging buffers)."""
+    cfg = systems.robertson_config(size=65536)
+    params = torch.from_numpy(cfg["params"]).cuda()
+    kw = dict(rtol=cfg["rtol"], atol=cfg["atol"], launch="plain")
+
+    def solve(busy):
+        times, y0 = cfg["t_span"].copy(), torch.from_numpy(cfg["y0"].copy())
+        if busy:
+            torch.cuda._sleep(100_000_000)
+        hist = rodas5P.solve(cfg["ode_fn"], y0, times, params, **kw)
+        times *= 0.5
+        y0.mul_(0.5)
+        return hist
+
+    expected = solve(busy=False)
+    torch.cuda.synchronize()
+    assert torch.equal(solve(busy=True), expected)
+    assert torch.equal(expected, rodas5P.solve(cfg["ode_fn"], torch.from_numpy(cfg["y0"]).cuda(), cfg["t_span"], params, **kw))
+    assert _native.stages_pageable_copies(0)
