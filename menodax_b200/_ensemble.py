@@ -123,6 +123,11 @@ def to_device(t, device):
     return t.to(device=device, non_blocking=not waits)
 
 
+def times_to_device(times, device):
+    """Save times on ``device``; unlike ``to_device``'s, page-locked ones may be changed at once too."""
+    return to_device(times.clone() if times.is_pinned() else times, device)
+
+
 @lru_cache(maxsize=None)
 def _staged_copies(index) -> bool:
     return _native.stages_pageable_copies(torch.cuda.current_device() if index is None else index)

@@ -36,7 +36,7 @@ from dataclasses import replace
 import torch
 
 from menodax_b200 import _native, autotune
-from menodax_b200._ensemble import initial_step, launch, pick_device, solver_stats, stream_key, to_device
+from menodax_b200._ensemble import initial_step, launch, pick_device, solver_stats, stream_key, times_to_device
 from menodax_b200._problem import get_problem
 
 # Checkpoint capacity (accepted steps per trajectory) and stride last used per
@@ -443,7 +443,7 @@ def solve_with_grad(ode_fn, y0, t_span, params, options, *, rtol, atol, first_st
     n_vars, n_params = y0_t.shape[1], p_t.shape[1]
     # Kept on the host too: the hints' keys read them without waiting for the device.
     times_h = torch.as_tensor(t_span, dtype=torch.float64).detach()
-    times = to_device(times_h, device)
+    times = times_to_device(times_h, device)
     if sens_param_columns is not None:
         cols = [int(c) for c in sens_param_columns]
         if len(set(cols)) != len(cols):

@@ -29,7 +29,7 @@ import numpy as np
 import torch
 
 from menodax_b200 import _native, autotune
-from menodax_b200._ensemble import initial_step, launch, normalize_y0_params, pick_device, stream_key, to_device
+from menodax_b200._ensemble import initial_step, launch, normalize_y0_params, pick_device, stream_key, times_to_device, to_device
 from menodax_b200._problem import KernelOptions, get_problem
 
 # Per joint-solve problem: the trajectories of the last call, longest first (by
@@ -158,7 +158,7 @@ def solve_joint(solver, ode_fn, y0, t_span, params, *, wrt_y0, wrt_params, sens_
         times_h = t_span.detach().to(torch.float64)
     else:
         times_h = torch.as_tensor(np.asarray(t_span, dtype=np.float64))
-    times = to_device(times_h, device)
+    times = times_to_device(times_h, device)
     # The persistent refill launch, trajectories longest first by the previous
     # call's step counts for the same problem: the joint solves are long and
     # uneven, and the order only moves when each trajectory runs (the 2-state

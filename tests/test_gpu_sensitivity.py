@@ -104,3 +104,30 @@ def test_joint_solve_visiting_order_changes_nothing():
     ordered = sensitivity.solve("rodas5P", cfg["ode_fn"], cfg["y0"], t_span, cfg["params"], **kw)
     for a, b in zip(first, ordered):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["sensitivities", "gradient"])
+def test_page_locked_save_times_may_change_as_soon_as_the_call_returns(kind):
+    """With the stream held up for some tens of milliseconds, the call returns before its
+    copies have run."""
+    cfg = systems.robertson_config(size=64)
+    y0, params = (torch.from_numpy(cfg[k]).cuda().requires_grad_(kind == "gradient") for k in ("y0", "params"))
+
+    def solve(busy):
+        times = torch.from_numpy(cfg["t_span"]).clone().pin_memory()
+        if busy:
+            torch.cuda._sleep(100_000_000)
+        if kind == "gradient":
+            hist = rodas5P.solve(cfg["ode_fn"], y0, times, params, rtol=1e-6, atol=1e-10)
+        else:
+            hist, _ = sensitivity.solve("rodas5P", cfg["ode_fn"], y0, times, params, rtol=1e-6, atol=1e-10)
+        times *= 0.5
+        return hist.detach()
+
+    expected = solve(busy=False)
+    torch.cuda.synchronize()
+    assert torch.equal(solve(busy=True), expected)
+    held = torch.from_numpy(cfg["t_span"]).cuda()
+    again = (rodas5P.solve(cfg["ode_fn"], y0, held, params, rtol=1e-6, atol=1e-10).detach() if kind == "gradient" else
+             sensitivity.solve("rodas5P", cfg["ode_fn"], y0, held, params, rtol=1e-6, atol=1e-10)[0])
+    assert torch.equal(expected, again)
