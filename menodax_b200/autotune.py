@@ -185,8 +185,10 @@ def streams_to_host(choice: LaunchChoice) -> bool:
     trajectory finished within the probe's step cap), where the history's trip
     across the host link takes longer than the kernel; the one-launch kernel's
     warps copy their rows to the host as they finish, which the persistent
-    launch cannot do in whole rows, so it gets the history there sooner."""
-    return choice.mode == _native.MDX_LAUNCH_PERSISTENT and choice.team == 0 and choice.grid_fill == 1.0
+    launch cannot do in whole rows, so it gets the history there sooner.  A staged
+    choice is for long integrations and stays, whatever its fill."""
+    return (choice.mode == _native.MDX_LAUNCH_PERSISTENT and choice.team == 0 and choice.grid_fill == 1.0
+            and not choice.staged)
 
 
 def longest_first(loop_steps: torch.Tensor) -> torch.Tensor:

@@ -67,6 +67,16 @@ def test_a_half_filled_persistent_launch_is_kept_and_copied_after_the_kernel(stu
     assert second["order"].numel() == 4096
 
 
+@pytest.mark.parametrize("fill", [0.5, 1.0])
+def test_a_staged_choice_runs_staged_for_host_results_too(stub_device, monkeypatch, fill):
+    """Never the one-launch kernel with a slice, which the launch refuses; no order goes in
+    and none is kept."""
+    _solve(monkeypatch, autotune.LaunchChoice(128, PERSISTENT, fill, 0, staged=True))
+    kw = stub_device[-1]
+    assert kw["mode"] == PERSISTENT and kw["slice_steps"] == autotune.STAGE_STEPS
+    assert kw["hist_host"] is None and kw["order"] is None and not _frontend._order_hint
+
+
 class HostTensor:
     """What ``to_device`` asks of a host tensor, and the copies it starts."""
 
