@@ -60,42 +60,19 @@ __device__ __forceinline__ double weight(const MdxSolveArgs& a, int traj, int j)
 }
 
 // Dense-output weights b1..b7 at theta (Tsitouras 2011 continuous extension,
-// modax/tsit5.py:307-344): theta times the cubic p0 + p1 theta + p2 theta^2 + p3 theta^3.
-// The factored forms of the tables are multiplied out at compile time and take three
-// multiply-adds each; with a few saves per trajectory most steps of a warp have a lane
-// that interpolates (Lorenz, 250,007 trajectories on a B200: with the kept first stage
-// and save time below, 903 -> 889 us a call).  factored_* give (p0, p1, p2, p3) of c (theta - r) (theta^2 - q
-// theta + w) and of c theta (theta - r) (theta - s).
-struct Cubic { double p[4]; };
-__host__ __device__ constexpr Cubic factored_first(double c, double r, double q, double w) {
-  return Cubic{{-c * r * w, c * (w + r * q), -c * (q + r), c}};
-}
-__host__ __device__ constexpr Cubic factored_quadratic(double c, double q, double w) {
-  return Cubic{{0.0, c * w, -c * q, c}};
-}
-__host__ __device__ constexpr Cubic factored_roots(double c, double r, double s) {
-  return factored_quadratic(c, r + s, r * s);
-}
-__host__ __device__ constexpr Cubic dense_cubic(int i) {
-  constexpr Cubic t[7] = {
-      factored_first(-1.0530884977290216, 1.3299890189751412, 1.4364028541716351, 0.7139816917074209),
-      factored_quadratic(0.1017, 2.1966568338249754, 1.2949852507374631),
-      factored_quadratic(2.490627285651252793, 2.38535645472061657, 1.57803468208092486),
-      factored_roots(-16.54810288924490272, 1.21712927295533244, 0.61620406037800089),
-      factored_roots(47.37952196282928122, 1.203071208372362603, 0.658047292653547382),
-      factored_roots(-34.87065786149660974, 1.2, 0.666666666666666667),
-      factored_roots(2.5, 1.0, 0.6),
-  };
-  return t[i];
-}
-
+// modax/tsit5.py:307-344), from the tables' factors: theta less a root is rounded once however
+// close they are, so a weight is good to a few roundings of itself.  Multiplied out to
+// powers of theta the same polynomials cost two operations a weight less and lose two digits
+// between their large coefficients (mean error of the weights' sum 4.2e-15 against 2e-16).
 __device__ __forceinline__ void dense_weights(double th, double b[7]) {
-#pragma unroll
-  for (int i = 0; i < 7; ++i) {
-    const Cubic c = dense_cubic(i);
-    const double tail = c.p[1] + th * (c.p[2] + th * c.p[3]);
-    b[i] = th * (i == 0 ? c.p[0] + th * tail : th * tail);
-  }
+  const double th2 = th * th;
+  b[0] = (-1.0530884977290216 * th) * ((th - 1.3299890189751412) * (th * (th - 1.4364028541716351) + 0.7139816917074209));
+  b[1] = (0.1017 * th2) * (th * (th - 2.1966568338249754) + 1.2949852507374631);
+  b[2] = (2.490627285651252793 * th2) * (th * (th - 2.38535645472061657) + 1.57803468208092486);
+  b[3] = (-16.54810288924490272 * th2) * ((th - 1.21712927295533244) * (th - 0.61620406037800089));
+  b[4] = (47.37952196282928122 * th2) * ((th - 1.203071208372362603) * (th - 0.658047292653547382));
+  b[5] = (-34.87065786149660974 * th2) * ((th - 1.2) * (th - 0.666666666666666667));
+  b[6] = (2.5 * th2) * ((th - 1.0) * (th - 0.6));
 }
 
 __device__ __forceinline__ void init(State& st, const MdxSolveArgs& a, int traj) {

@@ -448,3 +448,42 @@ def test_one_fast_reaction_takes_the_steps_of_a_double_lu(tmp_path, rate):
     assert (c[3] == 0).all()
     assert c[2].mean() <= 1.05 * c0[2].mean() + 1
     np.testing.assert_allclose(h, h0, rtol=2e-5, atol=1e-9)
+
+
+def test_tsit5_dense_output_weights_are_good_to_a_few_roundings(tmp_path):
+    """Against the tables' factored polynomials in rational numbers.  A weight is a product of
+    at most five factors; a distance to a root is rounded once, so a weight with real roots is
+    good to eight roundings of itself, one with a quadratic factor to eight of that factor's
+    terms."""
+    from fractions import Fraction as F
+
+    cfg = systems.lorenz_config(size=1)
+    source, _ = build_source(cfg["ode_fn"], 3, 1, KernelOptions(solver="tsit5"))
+    source = source.replace('#include "mdx_entry.cuh"', "")
+    probe = 'extern "C" void weights(double th, double* b) { mdx::tsit5::dense_weights(th, b); }'
+    cpp, so = tmp_path / "w.cpp", tmp_path / "w.so"
+    cpp.write_text(PRELUDE + THREAD_DIMS + source + probe)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", "-mfma", "-ffp-contract=fast", f"-I{KERNEL_DIR}",
+                    str(cpp), "-o", str(so)], check=True)
+    run = ctypes.CDLL(str(so)).weights
+    run.argtypes = [ctypes.c_double, ctypes.c_void_p]
+    roots = [(-16.54810288924490272, 1.21712927295533244, 0.61620406037800089),
+             (47.37952196282928122, 1.203071208372362603, 0.658047292653547382),
+             (-34.87065786149660974, 1.2, 0.666666666666666667), (2.5, 1.0, 0.6)]
+    quadratics = [(0.1017, 2.1966568338249754, 1.2949852507374631),
+                  (2.490627285651252793, 2.38535645472061657, 1.57803468208092486)]
+    got = np.empty(7)
+    for theta in np.concatenate([[1.0, 0.6, 0.99999, 0.5], np.random.default_rng(5).uniform(0.0, 1.0, 300)]):
+        run(theta, got.ctypes.data)
+        th = F(theta)
+        c, r, q, w = (F(v) for v in (-1.0530884977290216, 1.3299890189751412, 1.4364028541716351, 0.7139816917074209))
+        expected = [c * th * (th - r) * (th * (th - q) + w)]
+        size = [abs(c * th * (th - r)) * (th * abs(th - q) + w)]
+        for c, q, w in (map(F, row) for row in quadratics):
+            expected.append(c * th * th * (th * (th - q) + w))
+            size.append(abs(c) * th * th * (th * abs(th - q) + w))
+        for c, r, s in (map(F, row) for row in roots):
+            expected.append(c * th * th * (th - r) * (th - s))
+            size.append(abs(expected[-1]))
+        for b, e, m in zip(got, expected, size):
+            assert abs(F(float(b)) - e) <= 8 * F(2) ** -53 * m
