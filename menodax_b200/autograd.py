@@ -204,7 +204,8 @@ class _EnsembleSolve(torch.autograd.Function):
         kw = dict(y0=y0c, times=times, params=pc, weights=None, dt0=dt0, rtol=rtol, atol=atol,
                   max_steps=max_steps, mode=_native.MDX_LAUNCH_PERSISTENT)
         capacity, stride_hint = _capacity_hint.get(key, (None, None))
-        order = _order_hint.get(key)
+        order_key = (key, stream_key(y0.device))
+        order = _order_hint.get(order_key)
         if order is not None and (order.device != y0.device or order.numel() != n):
             order = None
         if capacity is None:
@@ -231,7 +232,7 @@ class _EnsembleSolve(torch.autograd.Function):
             capacity = int(needed * 1.1) + 8
             del ckpt
         _remember(_capacity_hint, key, (max(needed + 8, int(needed * 1.1)), stride))
-        _remember(_order_hint, key, autotune.longest_first(counters[0]))
+        _remember(_order_hint, order_key, autotune.longest_first(counters[0]))
         last_checkpoint.update(stride=stride, capacity=capacity, bytes=nbytes, forward_fill=fill)
         ctx.problem = problem
         ctx.capacity = capacity
@@ -460,8 +461,7 @@ def solve_with_grad(ode_fn, y0, t_span, params, options, *, rtol, atol, first_st
         keep[list(int(c) for c in sens_param_columns)] = 1.0
         p_t = _ColumnMask.apply(p_t, keep)
     problems = _Problems(ode_fn, n_vars, n_params, replace(options, runtime_weights=False))
-    key = (ode_fn, n_vars, n_params, options, n, tuple(times_h.tolist()), float(rtol), float(atol),
-           stream_key(device))
+    key = (ode_fn, n_vars, n_params, options, n, tuple(times_h.tolist()), float(rtol), float(atol))
     hist, counters = _EnsembleSolve.apply(y0_t, p_t, times, problems, initial_step(first_step), rtol,
                                           atol, max_steps, key)
     if return_stats:

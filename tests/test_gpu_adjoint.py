@@ -359,3 +359,38 @@ def test_forward_visiting_order_changes_nothing_but_the_schedule():
     plain = _grads(rodas5P.solve, cfg["ode_fn"], cfg["y0"], t_span, cfg["params"], w, **kw)
     for a, b in zip(ordered, plain):
         assert np.array_equal(a, b)
+
+
+def test_a_new_stream_needs_no_counting_solve(monkeypatch):
+    """What a call learns of the problem's step counts holds on every stream; only the visiting
+    order, a device tensor, is read where it was written."""
+    from menodax_b200 import autograd
+
+    cfg = systems.vdp_gradient_config(1, size=256)
+    times = np.linspace(0.0, 5.0, 4)
+    launches = []
+    launch = autograd.launch
+    monkeypatch.setattr(autograd, "launch", lambda *a, **k: launches.append(k["order"] is not None if "order" in k else False)
+                        or launch(*a, **k))
+    autograd._capacity_hint.clear()
+    autograd._order_hint.clear()
+
+    def gradient():
+        launches.clear()
+        y0 = torch.from_numpy(cfg["y0"]).cuda().requires_grad_()
+        params = torch.from_numpy(cfg["params"]).cuda().requires_grad_()
+        hist = rodas5P.solve(cfg["ode_fn"], y0, times, params, lu_precision="fp64", sens_error_control=False)
+        return torch.autograd.grad((hist ** 2).sum(), (y0, params))
+
+    first = gradient()
+    assert len(launches) == 2                    # the counting solve and the checkpointing one
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        again = gradient()
+        assert launches == [False]               # one, in index order
+        gradient()
+        assert launches == [True]
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(first, again))
+    autograd._capacity_hint.clear()
+    autograd._order_hint.clear()
