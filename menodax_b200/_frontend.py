@@ -145,7 +145,9 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
         streamed = mode == _native.MDX_LAUNCH_PLAIN
     order = None
     order_key = None
-    if mode == _native.MDX_LAUNCH_PERSISTENT and not slice_steps:
+    # A graph neither reads an order, which would be gone or another at its replay, nor leaves one,
+    # which nothing has written yet.
+    if mode == _native.MDX_LAUNCH_PERSISTENT and not slice_steps and not torch.cuda.is_current_stream_capturing():
         order_key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol),
                      int(max_steps), int(grid_blocks), stream_key(device))
         order = _order_hint.get(order_key)
