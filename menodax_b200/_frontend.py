@@ -47,6 +47,10 @@ def _remember_order(key, order) -> None:
         _order_hint.pop(next(iter(_order_hint)))
 
 
+def _capturing() -> bool:
+    return torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing()
+
+
 def _is_torch(*xs):
     return any(isinstance(x, torch.Tensor) for x in xs)
 
@@ -147,7 +151,7 @@ def run(ode_fn, y0, t_span, params, options: KernelOptions, *, rtol, atol, first
     order_key = None
     # A graph neither reads an order, which would be gone or another at its replay, nor leaves one,
     # which nothing has written yet.
-    if mode == _native.MDX_LAUNCH_PERSISTENT and not slice_steps and not torch.cuda.is_current_stream_capturing():
+    if mode == _native.MDX_LAUNCH_PERSISTENT and not slice_steps and not _capturing():
         order_key = (ode_fn, n_vars, n_params, options, n, tuple(times.tolist()), float(rtol), float(atol),
                      int(max_steps), int(grid_blocks), stream_key(device))
         order = _order_hint.get(order_key)

@@ -81,13 +81,13 @@ def test_a_captured_launch_neither_reads_nor_leaves_a_visiting_order(stub_device
     """A replay would read an order that is gone by then, and a later call one that no replay
     has written: indexes out of range either way."""
     choice = autotune.LaunchChoice(128, PERSISTENT, 0.5, 0)
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    monkeypatch.setattr(_frontend, "_capturing", lambda: True)
     _solve(monkeypatch, choice)
     assert stub_device[-1]["order"] is None and not _frontend._order_hint
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(_frontend, "_capturing", lambda: False)
     _solve(monkeypatch, choice)
     assert len(_frontend._order_hint) == 1
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    monkeypatch.setattr(_frontend, "_capturing", lambda: True)
     _solve(monkeypatch, choice)
     assert stub_device[-1]["mode"] == PERSISTENT and stub_device[-1]["order"] is None
 
