@@ -75,7 +75,8 @@ class KernelOptions:
     # registers (kernels/mdx_team_inverse.cuh) instead of factorised in shared memory.
     inverse: bool = False
     # A persistent launch in two stages (kernels/mdx_entry.cuh, mdx_solve_staged): thread and
-    # cyclic kernels of plain solves.
+    # cyclic kernels of plain solves.  The autotuner stages Rodas5P's; Tsit5's is for callers
+    # of the C ABI.
     staged: bool = False
     # Tsit5: the stage vectors k1..k6 in shared memory, one column per thread
     # (the reference's "shared" backend, modax/tsit5.py:117-139).
@@ -144,8 +145,9 @@ def closed_inverse(options: KernelOptions, n_vars: int) -> bool:
 def wide_solve(options: KernelOptions, n_vars: int) -> bool:
     """Whether a thread-kernel Rodas5P build solves its stages in double against
     FP32 factors: ``options.wide_solve`` when set, else for systems of at most
-    ``WIDE_SOLVE_MAX_VARS`` states (a joint sensitivity system follows its base
-    system, so its state rows match the plain solve's)."""
+    ``WIDE_SOLVE_MAX_VARS`` states.  A joint sensitivity system follows its base
+    system, so its state rows match the plain solve's, but for dense ones of up to
+    ``CLOSED_INVERSE_MAX`` states, whose plain solve inverts its matrix instead."""
     if not wide_solve_applies(options):
         return False
     if options.wide_solve is not None:

@@ -93,7 +93,11 @@ def solve(
     ``16`` or ``32`` give each trajectory a team of that many lanes with its
     vectors and matrix in shared memory; ``"auto"`` leaves the choice to the
     launch autotuner, which considers teams for systems of
-    ``autotune.TEAM_MIN_VARS`` or more states.  Teams run no forward
+    ``autotune.TEAM_MIN_VARS`` or more states, with fast FP32 LUs also teams that
+    keep a dense matrix's inverse in their registers and, for systems that repeat around
+    a ring and have a sparsity pattern, lanes that each keep a block of the state in theirs
+    (FP64 stage solves against FP32 factors, unpivoted as the sparse LU).  Ensembles
+    too small to tune take the one of these that ``autotune.small_choice`` names.  Teams run no forward
     sensitivities; a save hook runs on a team's first lane; with a sparsity pattern and
     ``sens_error_control=False`` a team also runs the discrete adjoint (its
     checkpointing forward pass and its reverse sweep).
