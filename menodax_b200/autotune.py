@@ -164,7 +164,7 @@ def grid_blocks(problem, choice: LaunchChoice, n: int) -> int:
 STAGE_STEPS = 128
 # Rings on a B200, in index order / staged: 8 states on threads, t in [0, 300] 35.1 /
 # 29.6 ms, [0, 3000] 287 / 253 (ordered by exact step counts 249); 32 states on cyclic
-# lanes, whose longest trajectories set the time in any order, 22.9 / 23.2.
+# lanes, whose longest trajectories set the time in any order, 24.1 / 24.1.
 STAGE_GAIN = 0.03
 
 
